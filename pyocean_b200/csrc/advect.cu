@@ -123,7 +123,7 @@ __device__ __forceinline__ void coeff_body(const StepArgs& a, int i, int j, int 
     const Shape s = a.s;
     const Flags fl(a.flags);
     if (i >= s.nx || j >= s.ny) return;
-    const double* cL = a.q1;
+    const double* cL = a.c1;
     // the 7-point stencil of the bounds: cell, x / y neighbours, layers k -+ 1 (ok cells only); its geometry is
     // the same for every tracer
     const int dk[7] = {0, 0, 0, 0, 0, -1, 1};
@@ -173,7 +173,7 @@ __device__ __forceinline__ void coeff_body(const StepArgs& a, int i, int j, int 
             rin = p_in > 0.0 ? pmin(1.0, q_in / p_in) : 0.0;
             rout = p_out > 0.0 ? pmin(1.0, q_out / p_out) : 0.0;
         }
-        a.c1[ci] = rin;            // R+ over c1
+        a.q1[ci] = rin;            // R+ (over the stencil classes)
         a.c2[ci] = rout;           // R- over c2
     }
 }
@@ -187,7 +187,7 @@ __device__ __forceinline__ double coef_x(const StepArgs& a, const Shape& s, cons
     if (fl.per_x) { l = wrap(l, s.nx); r = wrap(r, s.nx); }
     else if (f < 1 || f > s.nx - 1) return 0.0;
     const i64 ol = s.cell(t, k, j, l), orr = s.cell(t, k, j, r);
-    return A >= 0.0 ? pmin(a.c1[orr], a.c2[ol]) : pmin(a.c1[ol], a.c2[orr]);
+    return A >= 0.0 ? pmin(a.q1[orr], a.c2[ol]) : pmin(a.q1[ol], a.c2[orr]);
 }
 
 __device__ __forceinline__ double coef_y(const StepArgs& a, const Shape& s, const Flags& fl, int t, int k, int f,
@@ -197,7 +197,7 @@ __device__ __forceinline__ double coef_y(const StepArgs& a, const Shape& s, cons
     if (fl.per_y) { l = wrap(l, s.ny); r = wrap(r, s.ny); }
     else if (f < 1 || f > s.ny - 1) return 0.0;
     const i64 ol = s.cell(t, k, l, i), orr = s.cell(t, k, r, i);
-    return A >= 0.0 ? pmin(a.c1[orr], a.c2[ol]) : pmin(a.c1[ol], a.c2[orr]);
+    return A >= 0.0 ? pmin(a.q1[orr], a.c2[ol]) : pmin(a.q1[ol], a.c2[orr]);
 }
 
 // Pass 5: C_out = safe(q0 - dt div(F_L + C A), V1) (sigma_baroclinic.py:514-530).  One thread per column cell
@@ -247,7 +247,7 @@ __device__ __forceinline__ void final_body(const StepArgs& a, int i, int j, int 
         const int p = t * s.n + k;
         const i64 pc = plane_at(p, pl);
         const double* C = a.C + pc;
-        const double* Rp = a.c1 + pc;
+        const double* Rp = a.q1 + pc;
         const double* Rm = a.c2 + pc;
         const double c0 = __ldg(C + o_c), cw = __ldg(C + o_w), ce = __ldg(C + o_e), cs = __ldg(C + o_s),
                      cn = __ldg(C + o_n);
@@ -365,30 +365,82 @@ __global__ void __launch_bounds__(256) fct_open_flux_kernel(StepArgs a, double* 
 // SSP-RK3 without limiter (tracers.py:342-375): per stage a face pass (the x, y and z WENO5 faces of _advect_div)
 // and a cell pass (the stage update of _rk_stage).
 
+// One plane (t, k) of a face pass as pointers; element offsets are 32-bit.
+struct FacePlane {
+    const double* __restrict__ c;     // the field
+    const double* __restrict__ e;     // exterior on open edges (inflow, else the field)
+    const uint8_t* __restrict__ ok;
+    const double* __restrict__ qx;
+    const double* __restrict__ qy;
+};
+
+// WENO5 flux through the west x-face (f = i) of cell (j, i), 0 where Q = 0, and through the domain-edge faces
+// f = 0, nx of an axis that does not wrap (sigma_baroclinic.py:277-297); cls: the face's two classes.
+template <bool ZV>
+__device__ __forceinline__ double x_flux(const FacePlane& P, const Shape& s, const Flags& fl, int j, int f,
+                                         unsigned cls)
+{
+    const int o = j * s.nx + f;
+    const double q = __ldg(P.qx + (o + j));
+    if (fl.per_x || (f >= 1 && f <= s.nx - 1)) {
+        if (q == 0.0) return 0.0;
+        const bool pos = q >= 0.0;
+        return q * face_value<ZV, false, false>(P.c, o, 1, s.nx, fl.per_x, f, pos, (pos ? cls : cls >> 2) & 3u);
+    }
+    if (f == 0) return fl.open_w ? q * (q > 0.0 ? P.e[o] : P.c[o]) : 0.0;
+    return fl.open_e ? q * (q < 0.0 ? P.e[o - 1] : P.c[o - 1]) : 0.0;
+}
+
+// The same for the south y-face (f = j) of cell (j, i).
+template <bool ZV>
+__device__ __forceinline__ double y_flux(const FacePlane& P, const Shape& s, const Flags& fl, int f, int i,
+                                         unsigned cls)
+{
+    const int o = f * s.nx + i;
+    const double q = __ldg(P.qy + o);
+    if (fl.per_y || (f >= 1 && f <= s.ny - 1)) {
+        if (q == 0.0) return 0.0;
+        const bool pos = q >= 0.0;
+        return q * face_value<ZV, false, false>(P.c, o, s.nx, s.ny, fl.per_y, f, pos, (pos ? cls : cls >> 2) & 3u);
+    }
+    if (f == 0) return fl.open_s ? q * (q > 0.0 ? P.e[o] : P.c[o]) : 0.0;
+    return fl.open_n ? q * (q < 0.0 ? P.e[o - s.nx] : P.c[o - s.nx]) : 0.0;
+}
+
 // z-face flux through interface kf (between layers kf-1 and kf) of column (j, i): WENO5 in k on the layers of the
 // column, valid cells only, 0 on the bed and surface interfaces (sigma_baroclinic.py:335-353).
-__device__ __forceinline__ double zface_flux(const StepArgs& a, const Shape& s, const Flags& fl, const double* cin,
-                                             int t, int kf, int j, int i)
+template <bool ZV>
+__device__ __forceinline__ double z_flux(const StepArgs& a, const Shape& s, const double* cin, int t, int kf, int ij,
+                                         unsigned cls)
 {
     if (a.Fz == nullptr || kf < 1 || kf > s.n - 1) return 0.0;
-    const int pl = s.ny * s.nx, ij = j * s.nx + i;            // 32-bit offsets within a field
+    const int pl = s.ny * s.nx;                               // 32-bit offsets within a field
     const double q = a.Fz[kf * pl + ij];
     if (q == 0.0) return 0.0;
-    const double* ct = cin + plane_at(t, s.n * pl);
-    // the five upwind layers in upwind order, as the reference passes them to _wval: kf-3 .. kf+1 when q >= 0,
-    // kf+2 .. kf-2 when q < 0 (no per-value selects)
     const bool pos = q >= 0.0;
-    const int k0 = pos ? kf - 3 : kf + 2, dk = pos ? 1 : -1;
-    double w[5];
-    bool v[5];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-        const int kk = k0 + m * dk;
-        const bool in = kk >= 0 && kk < s.n;
-        w[m] = in ? ct[kk * pl + ij] : 0.0;
-        v[m] = in && a.ok[(in ? kk : 0) * pl + ij] != 0;
-    }
-    return q * weno5_value(w[0], w[1], w[2], w[3], w[4], v[0], v[1], v[2], v[3], v[4], fl.z);
+    return q * face_value<ZV, false, false>(cin + plane_at(t, s.n * pl), kf * pl + ij, pl, s.n, false, kf, pos,
+                                     (pos ? cls : cls >> 2) & 3u);
+}
+
+// Classes of the three faces of cell (k, j, i) (see face_class): bits 0-3 west, 4-7 south, 8-11 bottom.
+__device__ __forceinline__ unsigned rk3_classes(const StepArgs& a, const Shape& s, const Flags& fl, int k, int j, int i)
+{
+    const int pl = s.ny * s.nx, ij = j * s.nx + i;
+    const uint8_t* ok = a.ok + plane_at(k, pl);
+    unsigned c = line_class(ok + j * s.nx, 1, s.nx, fl.per_x, i) | line_class(ok + i, s.nx, s.ny, fl.per_y, j) << 4;
+    if (a.Fz != nullptr) c |= line_class(a.ok + ij, pl, s.n, false, k) << 8;
+    return c;
+}
+
+// Class pass of the unlimited WENO5 step: one thread per cell, once for the step's face passes and tracers.
+template <int TJR>
+__global__ void __launch_bounds__(TI * TJR) rk3_class_kernel(StepArgs a, uint16_t* __restrict__ cls)
+{
+    const Shape s = a.s;
+    const Flags fl(a.flags);
+    const int i = blockIdx.x * TI + threadIdx.x % TI, j = blockIdx.y * TJR + threadIdx.x / TI, k = blockIdx.z;
+    if (i >= s.nx || j >= s.ny) return;
+    cls[plane_at(k, s.ny * s.nx) + (j * s.nx + i)] = (uint16_t)rk3_classes(a, s, fl, k, j, i);
 }
 
 // Face values of the reference's NumPy RHS (tracers.py:110-151), used by `advect` for the upwind-3 / upwind-1
@@ -492,15 +544,17 @@ __device__ __forceinline__ double zface_lin(const StepArgs& a, const Shape& s, c
 // A single kernel per stage on shared-memory tiles, which computed every z-face twice (once for each of its two
 // cells), took 6.68 ms at 512 x 512 x 50 with a vertical transport; these passes take 3.86 ms, bit-identical.
 // Stages 1-3: SSP-RK3 (input C, c1, c2); 4: the 'pc' predictor (input C, centred faces, half step to c1); 5: the
-// 'pc' corrector (input c1, the scheme's faces, full step from C).
+// 'pc' corrector (input c1, the scheme's faces, full step from C); 0: one evaluation of C's faces.  The WENO5 faces of
+// the steps read their stencils' classes from `cls` (rk3_class_kernel); the single evaluation works its own out.
 template <int STAGE>
 __device__ __forceinline__ const double* rk3_stage_field(const StepArgs& a)
 {
-    return (STAGE == 1 || STAGE == 4) ? a.C : ((STAGE == 2 || STAGE == 5) ? a.c1 : a.c2);
+    return (STAGE <= 1 || STAGE == 4) ? a.C : ((STAGE == 2 || STAGE == 5) ? a.c1 : a.c2);
 }
 
 template <int STAGE, bool ZV, int FS>
-__device__ __forceinline__ void rk3_faces_body(const StepArgs& a, int t, int k, int i, int j)
+__device__ __forceinline__ void rk3_faces_body(const StepArgs& a, const uint16_t* __restrict__ classes, int t, int k,
+                                               int i, int j)
 {
     const Shape s = a.s;
     const Flags fl(a.flags);
@@ -511,14 +565,12 @@ __device__ __forceinline__ void rk3_faces_body(const StepArgs& a, int t, int k, 
     FacePlane P;
     P.c = cin + pc;
     P.e = a.inflow ? a.inflow + pc : P.c;
-    P.c0 = P.c;
-    P.e0 = P.e;
     P.ok = a.ok + plane_at(k, pl);
     P.qx = a.Qx + plane_at(k, xpl);
     P.qy = a.Qy + plane_at(k, ypl);
     double* sx = a.Sx + plane_at(p, xpl);
     double* sy = a.Sy + plane_at(p, ypl);
-    const int fxo = j * (s.nx + 1) + i, fyo = j * s.nx + i;
+    const int fyo = j * s.nx + i, fxo = fyo + j;
     if (FS != FS_WENO) {
         sx[fxo] = x_face_lin<FS>(P, s, fl, j, i);
         sy[fyo] = y_face_lin<FS>(P, s, fl, j, i);
@@ -527,19 +579,21 @@ __device__ __forceinline__ void rk3_faces_body(const StepArgs& a, int t, int k, 
         if (j == s.ny - 1) sy[fyo + s.nx] = y_face_lin<FS>(P, s, fl, s.ny, i);
         return;
     }
-    double F, unused;
-    x_face<ZV, false, false>(P, s, fl, j, i, F, unused);
-    sx[fxo] = F;
-    y_face<ZV, false, false>(P, s, fl, j, i, F, unused);
-    sy[fyo] = F;
-    a.Tx[pc + fyo] = zface_flux(a, s, fl, cin, t, k, j, i);          // bottom interface k (0 at the bed)
-    if (i == s.nx - 1) {
-        x_face<ZV, false, false>(P, s, fl, j, s.nx, F, unused);
-        sx[fxo + 1] = F;
+    const unsigned cls = STAGE == 0 ? rk3_classes(a, s, fl, k, j, i) : __ldg(classes + plane_at(k, pl) + fyo);
+    const double fx = x_flux<ZV>(P, s, fl, j, i, cls);
+    sx[fxo] = fx;
+    if (fl.per_x && i == 0) sx[fxo + s.nx] = fx;                      // face nx of a periodic axis is face 0
+    const double fy = y_flux<ZV>(P, s, fl, j, i, cls >> 4);
+    sy[fyo] = fy;
+    if (fl.per_y && j == 0) sy[fyo + pl] = fy;
+    a.Tx[pc + fyo] = z_flux<ZV>(a, s, cin, t, k, fyo, cls >> 8);      // bottom interface k (0 at the bed)
+    if (i == s.nx - 1 && !fl.per_x) {
+        const double q = __ldg(P.qx + fxo + 1);
+        sx[fxo + 1] = fl.open_e ? q * (q < 0.0 ? P.e[fyo] : P.c[fyo]) : 0.0;
     }
-    if (j == s.ny - 1) {
-        y_face<ZV, false, false>(P, s, fl, s.ny, i, F, unused);
-        sy[fyo + s.nx] = F;
+    if (j == s.ny - 1 && !fl.per_y) {
+        const double q = __ldg(P.qy + fyo + s.nx);
+        sy[fyo + s.nx] = fl.open_n ? q * (q < 0.0 ? P.e[fyo] : P.c[fyo]) : 0.0;
     }
 }
 
@@ -549,11 +603,11 @@ __device__ __forceinline__ void rk3_faces_body(const StepArgs& a, int t, int k, 
 #define POCEAN_RK3_FACES_MINB 6
 #endif
 template <int STAGE, bool ZV, int FS, int TJR>
-__global__ void __launch_bounds__(TI * TJR, POCEAN_RK3_FACES_MINB * 256 / (TI * TJR)) rk3_faces_kernel(StepArgs a)
+__global__ void __launch_bounds__(TI * TJR, POCEAN_RK3_FACES_MINB * 256 / (TI * TJR)) rk3_faces_kernel(StepArgs a, const uint16_t* __restrict__ classes)
 {
     int k, t;
     split_plane(blockIdx.z, a.s.nt, a.tdiv, k, t);
-    rk3_faces_body<STAGE, ZV, FS>(a, t, k, blockIdx.x * TI + threadIdx.x % TI,
+    rk3_faces_body<STAGE, ZV, FS>(a, classes, t, k, blockIdx.x * TI + threadIdx.x % TI,
                                   blockIdx.y * TJR + threadIdx.x / TI);
 }
 
@@ -622,11 +676,7 @@ __device__ __forceinline__ double any_x_face(const FacePlane& P, const StepArgs&
                                              int k, int j, int f)
 {
     if (KIND == FACES_DONOR) return donor_x(P.c, P.e, a.Qx, s, fl, k, j, f);
-    if (KIND == FS_WENO) {
-        double F, unused;
-        x_face<ZV, false, false>(P, s, fl, j, f, F, unused);
-        return F;
-    }
+    if (KIND == FS_WENO) return x_flux<ZV>(P, s, fl, j, f, line_class(P.ok + j * s.nx, 1, s.nx, fl.per_x, f));
     return x_face_lin<KIND>(P, s, fl, j, f);
 }
 
@@ -635,11 +685,7 @@ __device__ __forceinline__ double any_y_face(const FacePlane& P, const StepArgs&
                                              int k, int f, int i)
 {
     if (KIND == FACES_DONOR) return donor_y(P.c, P.e, a.Qy, s, fl, k, f, i);
-    if (KIND == FS_WENO) {
-        double F, unused;
-        y_face<ZV, false, false>(P, s, fl, f, i, F, unused);
-        return F;
-    }
+    if (KIND == FS_WENO) return y_flux<ZV>(P, s, fl, f, i, line_class(P.ok + i, s.nx, s.ny, fl.per_y, f));
     return y_face_lin<KIND>(P, s, fl, f, i);
 }
 
@@ -658,8 +704,6 @@ __global__ void __launch_bounds__(TI * TJ) helper_faces_kernel(StepArgs a, doubl
     FacePlane P;
     P.c = a.C + pc;
     P.e = a.inflow ? a.inflow + pc : P.c;
-    P.c0 = P.c;
-    P.e0 = P.e;
     P.ok = a.ok + plane_at(k, pl);
     P.qx = a.Qx + plane_at(k, xpl);
     P.qy = a.Qy + plane_at(k, ypl);
@@ -769,21 +813,50 @@ static int common_checks(const char* fn, const void* C, const void* V0, const vo
 #define POCEAN_FACE_ROWS 8
 #endif
 
-template <bool ZV, bool MIX>
-static void launch_split(const StepArgs& a, int stage, cudaStream_t st, int nlayers = -1)
+// Whether the face CTAs of nl layers take one tracer each.  A thread that goes through every tracer of its cell pays
+// for its set-up, transports and stencil classes once (advect_fct at 512 x 512 x 50: 7 % faster with two tracers, 19 %
+// with four at reduced precision), but there are nt times fewer CTAs: below two per slot of the chip (148 SMs of eight 256-thread
+// CTAs) the planes' own CTAs fill it better.
+static int one_tracer_ctas(const Shape& s, int nl)
+{
+    const i64 tiles = (i64)ceil_div(s.nx, TI) * ceil_div(s.ny, POCEAN_FACE_ROWS) * nl;
+    return s.nt > 1 && tiles < 2 * 148 * 8;
+}
+
+static void launch_classes(const StepArgs& a, cudaStream_t st, int nl)
 {
     constexpr int R = POCEAN_FACE_ROWS;
-    const Shape& s = a.s;
-    const dim3 grid(ceil_div(s.nx, TI), ceil_div(s.ny, R), s.nt * (nlayers < 0 ? s.n : nlayers));
+    fct_class_kernel<R><<<dim3(ceil_div(a.s.nx, 4 * TI), ceil_div(a.s.ny, R), nl), TI * R, 0, st>>>(a);
+}
+
+// The face and cell passes of one stage over nl layers from a.k0 on.
+template <bool ZV, bool MIX>
+static void launch_split(const StepArgs& a, int stage, cudaStream_t st, int nl)
+{
+    constexpr int R = POCEAN_FACE_ROWS;
+    const dim3 grid(ceil_div(a.s.nx, TI), ceil_div(a.s.ny, R), a.s.nt * nl);
+    const dim3 fgrid(grid.x, grid.y, a.per_plane ? grid.z : nl);
     if (stage == 1) {
-        fct_faces_kernel<1, ZV, MIX, R><<<grid, TI * R, 0, st>>>(a);
+        fct_faces_kernel<1, ZV, MIX, R><<<fgrid, TI * R, 0, st>>>(a);
         fct_update_kernel<1, R><<<grid, TI * R, 0, st>>>(a);
     } else if (stage == 2) {
-        fct_faces_kernel<2, ZV, MIX, R><<<grid, TI * R, 0, st>>>(a);
+        fct_faces_kernel<2, ZV, MIX, R><<<fgrid, TI * R, 0, st>>>(a);
         fct_update_kernel<2, R><<<grid, TI * R, 0, st>>>(a);
-    } else {
-        fct_faces3_kernel<ZV, MIX, R><<<grid, TI * R, 0, st>>>(a);
+    } else if (stage == 3) {
+        fct_faces3_kernel<ZV, MIX, R><<<fgrid, TI * R, 0, st>>>(a);
+    } else {                                          // 4: the unlimited step's RK3 flux and final update
+        fct_faces_kernel<4, ZV, MIX, R><<<fgrid, TI * R, 0, st>>>(a);
+        fct_update_kernel<4, R><<<grid, TI * R, 0, st>>>(a);
     }
+}
+
+static void launch_stage(const StepArgs& a, bool mixed, int stage, cudaStream_t st, int nl)
+{
+    const bool zv = !(a.flags & POCEAN_WENO_JS);
+    if (zv && !mixed) launch_split<true, false>(a, stage, st, nl);
+    else if (!zv && !mixed) launch_split<false, false>(a, stage, st, nl);
+    else if (zv) launch_split<true, true>(a, stage, st, nl);
+    else launch_split<false, true>(a, stage, st, nl);
 }
 
 // The FCT step with FP64 (mixed = false) or FP32-weight (mixed = true) WENO faces; everything else FP64.
@@ -810,27 +883,15 @@ static int advect_fct_impl(const char* fn, bool mixed, const double* C, const do
     carve_fct_workspace(a, workspace);
     a.out = C_out; a.face_i = face_i; a.fx_face = fx_face;
 
-    const dim3 grid(ceil_div(nx, TI), ceil_div(ny, TJ), nt * nz);
-    const bool zv = !(flags & POCEAN_WENO_JS);
-    auto stage_passes = [&](int stage) {
-        if (zv && !mixed) launch_split<true, false>(a, stage, st);
-        else if (!zv && !mixed) launch_split<false, false>(a, stage, st);
-        else if (zv) launch_split<true, true>(a, stage, st);
-        else launch_split<false, true>(a, stage, st);
-    };
-    stage_passes(1);
-    stage_passes(2);
+    a.per_plane = one_tracer_ctas(a.s, nz);
+    launch_classes(a, st, nz);
+    launch_stage(a, mixed, 1, st, nz);
+    launch_stage(a, mixed, 2, st, nz);
     if (flags & POCEAN_FCT_UNLIMITED) {
-        constexpr int R = POCEAN_FACE_ROWS;
-        const dim3 g2(ceil_div(nx, TI), ceil_div(ny, R), nt * nz);
-        if (zv && !mixed) fct_faces_kernel<4, true, false, R><<<g2, TI * R, 0, st>>>(a);
-        else if (!zv && !mixed) fct_faces_kernel<4, false, false, R><<<g2, TI * R, 0, st>>>(a);
-        else if (zv) fct_faces_kernel<4, true, true, R><<<g2, TI * R, 0, st>>>(a);
-        else fct_faces_kernel<4, false, true, R><<<g2, TI * R, 0, st>>>(a);
-        fct_update_kernel<4, R><<<g2, TI * R, 0, st>>>(a);
+        launch_stage(a, mixed, 4, st, nz);
         return pocean_check_launch(fn);
     }
-    stage_passes(3);
+    launch_stage(a, mixed, 3, st, nz);
     fct_coeff_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nz), NTHREADS, 0, st>>>(a);
     fct_final_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nz), NTHREADS, 0, st>>>(a);
     if (fx_face) {
@@ -845,13 +906,14 @@ namespace po {
 
 // The FCT passes of every domain of a batch, one launch per pass (off_host: the CTA offsets also held on the device).
 template <bool ZV, bool MIX, int TJR>
-static void fct_batched_stages(const BatchDomain* doms, const int* po, unsigned np, int ndom, cudaStream_t st)
+static void fct_batched_stages(const BatchDomain* doms, const int* po, unsigned np, const int* lo, unsigned nl, int ndom,
+                               cudaStream_t st)
 {
-    fct_faces_batched<1, ZV, MIX, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
+    fct_faces_batched<1, ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
     fct_update_batched<1, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
-    fct_faces_batched<2, ZV, MIX, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
+    fct_faces_batched<2, ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
     fct_update_batched<2, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
-    fct_faces3_batched<ZV, MIX, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
+    fct_faces3_batched<ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
 }
 
 // The FCT passes of every domain of a batch, one launch per pass (off_host: the CTA offsets also held on the device).
@@ -860,12 +922,15 @@ static void fct_batched_impl(const BatchDomain* doms, const int* off_dev, const 
                              cudaStream_t st)
 {
     const int* po = off_dev + BP_PTILE * (ndom + 1);
+    const int* lo = off_dev + BP_LTILE * (ndom + 1);
     const int* to = off_dev + BP_TILE * (ndom + 1);
     const unsigned np = (unsigned)off_host[BP_PTILE * (ndom + 1) + ndom];
+    const unsigned nl = (unsigned)off_host[BP_LTILE * (ndom + 1) + ndom];
     const unsigned nt = (unsigned)off_host[BP_TILE * (ndom + 1) + ndom];
-    if (tile_rows == 4) fct_batched_stages<ZV, MIX, 4>(doms, po, np, ndom, st);
-    else if (tile_rows == 16) fct_batched_stages<ZV, MIX, 16>(doms, po, np, ndom, st);
-    else fct_batched_stages<ZV, MIX, 8>(doms, po, np, ndom, st);
+    fct_class_batched<<<nt, NTHREADS / 4, 0, st>>>(doms, to, ndom);
+    if (tile_rows == 4) fct_batched_stages<ZV, MIX, 4>(doms, po, np, lo, nl, ndom, st);
+    else if (tile_rows == 16) fct_batched_stages<ZV, MIX, 16>(doms, po, np, lo, nl, ndom, st);
+    else fct_batched_stages<ZV, MIX, 8>(doms, po, np, lo, nl, ndom, st);
     fct_coeff_batched<<<nt, NTHREADS, 0, st>>>(doms, to, ndom);
     fct_final_batched<<<nt, NTHREADS, 0, st>>>(doms, to, ndom);
 }
@@ -879,11 +944,11 @@ void fct_batched_launch(const BatchDomain* doms, const int* off_dev, const int* 
     else fct_batched_impl<false, true>(doms, off_dev, off_host, ndom, tile_rows, st);
 }
 
-// CTAs of each batched FCT pass for one domain: 32 x tile_rows tiles x planes (stage passes); 32 x 8 tiles x
-// layers (coefficient and final passes).
-void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& tile_ctas)
+// CTAs of each batched FCT pass for one domain (see BatchPass).
+void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& layer_ctas, int& tile_ctas)
 {
-    plane_ctas = ceil_div(s.nx, TI) * ceil_div(s.ny, tile_rows) * s.nt * s.n;
+    layer_ctas = ceil_div(s.nx, TI) * ceil_div(s.ny, tile_rows) * s.n;
+    plane_ctas = layer_ctas * s.nt;
     tile_ctas = ceil_div(s.nx, TI) * ceil_div(s.ny, TJ) * s.n;
 }
 
@@ -914,21 +979,22 @@ extern "C" int pocean_advect_fct_mixed(const double* C, const double* V0, const 
 // The passes of `advect`: three SSP-RK3 stages, or the 'pc' predictor (centred faces) and corrector (the
 // scheme's faces).
 template <bool ZV, int FS>
-static void launch_rk3(const StepArgs& a, bool pc, dim3 grid, cudaStream_t st)
+static void launch_rk3(const StepArgs& a, uint16_t* cls, bool pc, dim3 grid, cudaStream_t st)
 {
     constexpr int R = POCEAN_FACE_ROWS;
+    if (FS == FS_WENO) rk3_class_kernel<R><<<dim3(grid.x, grid.y, a.s.n), TI * R, 0, st>>>(a, cls);
     if (pc) {
-        rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a);
+        rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a, cls);
         rk3_update_kernel<4, R><<<grid, TI * R, 0, st>>>(a);
-        rk3_faces_kernel<5, ZV, FS, R><<<grid, TI * R, 0, st>>>(a);
+        rk3_faces_kernel<5, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
         rk3_update_kernel<5, R><<<grid, TI * R, 0, st>>>(a);
         return;
     }
-    rk3_faces_kernel<1, ZV, FS, R><<<grid, TI * R, 0, st>>>(a);
+    rk3_faces_kernel<1, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<1, R><<<grid, TI * R, 0, st>>>(a);
-    rk3_faces_kernel<2, ZV, FS, R><<<grid, TI * R, 0, st>>>(a);
+    rk3_faces_kernel<2, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<2, R><<<grid, TI * R, 0, st>>>(a);
-    rk3_faces_kernel<3, ZV, FS, R><<<grid, TI * R, 0, st>>>(a);
+    rk3_faces_kernel<3, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<3, R><<<grid, TI * R, 0, st>>>(a);
 }
 
@@ -956,7 +1022,8 @@ extern "C" int pocean_advect_rk3_f64(const double* C, const double* V0, const do
     const size_t cells = align_up((size_t)nt * nz * ny * nx * sizeof(double));
     a.q1 = (double*)w; w += cells;
     a.c1 = (double*)w; w += cells;
-    a.q2 = (double*)w; w += cells;
+    a.q2 = a.q1;                                       // stage 2 reads its cell's q1 before it writes q2 there
+    uint16_t* cls = (uint16_t*)w; w += cells;
     a.c2 = (double*)w; w += cells;
     a.tef0 = (double*)w; w += align_up((size_t)nt * nz * ny * sizeof(double));
     a.tef1 = (double*)w; w += align_up((size_t)nt * nz * ny * sizeof(double));
@@ -967,10 +1034,10 @@ extern "C" int pocean_advect_rk3_f64(const double* C, const double* V0, const do
     a.Sy = (double*)w;
     const dim3 grid(ceil_div(nx, TI), ceil_div(ny, POCEAN_FACE_ROWS), nt * nz);
     const bool pc = flags & POCEAN_TIME_PC;
-    if (flags & POCEAN_FACES_UP3) launch_rk3<false, FS_UP3>(a, pc, grid, st);
-    else if (flags & POCEAN_FACES_UP1) launch_rk3<false, FS_UP1>(a, pc, grid, st);
-    else if (flags & POCEAN_WENO_JS) launch_rk3<false, FS_WENO>(a, pc, grid, st);
-    else launch_rk3<true, FS_WENO>(a, pc, grid, st);
+    if (flags & POCEAN_FACES_UP3) launch_rk3<false, FS_UP3>(a, cls, pc, grid, st);
+    else if (flags & POCEAN_FACES_UP1) launch_rk3<false, FS_UP1>(a, cls, pc, grid, st);
+    else if (flags & POCEAN_WENO_JS) launch_rk3<false, FS_WENO>(a, cls, pc, grid, st);
+    else launch_rk3<true, FS_WENO>(a, cls, pc, grid, st);
     return pocean_check_launch(fn);
 }
 
@@ -1057,11 +1124,11 @@ extern "C" int pocean_advect_rhs_f64(const double* c, const double* Qx, const do
     constexpr int R = POCEAN_FACE_ROWS;
     const dim3 grid(ceil_div(nx, TI), ceil_div(ny, R), nt * nz);
     cudaStream_t st = (cudaStream_t)stream;
-    if (centred) rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a);
-    else if (flags & POCEAN_FACES_UP3) rk3_faces_kernel<1, false, FS_UP3, R><<<grid, TI * R, 0, st>>>(a);
-    else if (flags & POCEAN_FACES_UP1) rk3_faces_kernel<1, false, FS_UP1, R><<<grid, TI * R, 0, st>>>(a);
-    else if (flags & POCEAN_WENO_JS) rk3_faces_kernel<1, false, FS_WENO, R><<<grid, TI * R, 0, st>>>(a);
-    else rk3_faces_kernel<1, true, FS_WENO, R><<<grid, TI * R, 0, st>>>(a);
+    if (centred) rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a, nullptr);
+    else if (flags & POCEAN_FACES_UP3) rk3_faces_kernel<1, false, FS_UP3, R><<<grid, TI * R, 0, st>>>(a, nullptr);
+    else if (flags & POCEAN_FACES_UP1) rk3_faces_kernel<1, false, FS_UP1, R><<<grid, TI * R, 0, st>>>(a, nullptr);
+    else if (flags & POCEAN_WENO_JS) rk3_faces_kernel<0, false, FS_WENO, R><<<grid, TI * R, 0, st>>>(a, nullptr);
+    else rk3_faces_kernel<0, true, FS_WENO, R><<<grid, TI * R, 0, st>>>(a, nullptr);
     helper_rhs_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nt * nz), NTHREADS, 0, st>>>(a, rhs);
     return pocean_check_launch(fn);
 }
@@ -1097,13 +1164,9 @@ extern "C" int pocean_advect_fct_layers(int mixed, const double* C, const double
     a.k0 = k0;
     const int nl = k1 - k0;
     if (part == 0) {
-        const bool zv = !(flags & POCEAN_WENO_JS);
-        for (int stage = 1; stage <= 3; ++stage) {
-            if (zv && !mixed) launch_split<true, false>(a, stage, st, nl);
-            else if (!zv && !mixed) launch_split<false, false>(a, stage, st, nl);
-            else if (zv) launch_split<true, true>(a, stage, st, nl);
-            else launch_split<false, true>(a, stage, st, nl);
-        }
+        a.per_plane = one_tracer_ctas(a.s, nl);
+        launch_classes(a, st, nl);
+        for (int stage = 1; stage <= 3; ++stage) launch_stage(a, mixed != 0, stage, st, nl);
     } else {
         fct_coeff_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nl), NTHREADS, 0, st>>>(a);
         fct_final_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nl), NTHREADS, 0, st>>>(a);

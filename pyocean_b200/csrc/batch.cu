@@ -47,7 +47,7 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     std::vector<int> off((size_t)BP_COUNT * (ndom + 1), 0);
     const bool zv = !(domains[0].flags & POCEAN_WENO_JS);
     int nmax = 1;
-    long long tot[BP_COUNT] = {0, 0, 0, 0, 0, 0};
+    long long tot[BP_COUNT] = {};
     for (int d = 0; d < ndom; ++d) {
         const pocean_domain& D = domains[d];
         if (D.nt < 1 || D.nz < 1 || D.ny < 1 || D.nx < 1 || (long long)D.nt * D.nz > 65535 || D.nz > 256)
@@ -81,11 +81,11 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
             B.a.out = D.C_adv;
             B.h_src = D.h_src; B.h_tgt = D.h_tgt; B.wet = D.wet; B.remap_scheme = D.remap_scheme;
             B.rout = parity == 0 ? D.C_next : const_cast<double*>(D.C);
-            int sc, tc;
-            fct_batched_ctas(B.a.s, tile_rows, sc, tc);
+            int pc, lc, tc;
+            fct_batched_ctas(B.a.s, tile_rows, pc, lc, tc);
             if (parity == 0) {
                 const long long cb = ((long long)D.ny * D.nx + 127) / 128;
-                const long long n_pass[BP_COUNT] = {sc, tc, cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt, cb * D.nt};
+                const long long n_pass[BP_COUNT] = {pc, lc, tc, cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt, cb * D.nt};
                 for (int q = 0; q < BP_COUNT; ++q) {
                     off[(size_t)q * (ndom + 1) + d] = (int)tot[q];
                     tot[q] += n_pass[q];

@@ -42,6 +42,8 @@ struct StepArgs {
     int face_i;
     int k0;                             // first layer of a layer-range launch of the single-domain passes (else 0)
     unsigned tdiv;                      // plane_magic(s.nt): plane index -> layer without an integer division
+    int per_plane;                      // single-domain face CTAs take one (tracer, layer) plane each (split_tracers)
+    int pad_;                           // (copied in 8-byte words)
     double* fx_face;
 };
 
@@ -66,7 +68,13 @@ __device__ __forceinline__ void split_plane(int p, int nt, unsigned tdiv, int& k
 }
 
 // CTA offsets of every batched pass: domain d owns CTAs off[d] .. off[d+1]-1 of the launch (ndom + 1 entries each).
-enum BatchPass { BP_PTILE = 0, BP_TILE = 1, BP_RPAIR = 2, BP_RREM = 3, BP_RALL = 4, BP_RGEN = 5, BP_COUNT = 6 };
+enum BatchPass {
+    BP_PTILE = 0,       // tile_rows tiles of the (tracer, layer) planes: cell passes
+    BP_LTILE,           // tile_rows tiles of the layers: face passes
+    BP_TILE,            // 8-row tiles of the layers: class, coefficient and final passes
+    BP_RPAIR, BP_RREM, BP_RALL, BP_RGEN,
+    BP_COUNT
+};
 
 // The domain whose CTA range holds CTA b (binary search of off[0..ndom]).
 __device__ __forceinline__ int find_domain(const int* __restrict__ off, int ndom, int b)
@@ -100,7 +108,7 @@ void carve_fct_workspace(StepArgs& a, void* workspace);
 // Host launchers of the batched passes (advect.cu, remap.cu).
 void fct_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, bool zv,
                         bool mixed, int tile_rows, cudaStream_t st);
-void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& tile_ctas);
+void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& layer_ctas, int& tile_ctas);
 void remap_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int nf_mode,
                           int nmax, cudaStream_t st);
 

@@ -18,6 +18,9 @@
 
 namespace po {
 
+// The stencil classes of the domain's faces, one byte per cell, in the buffer that R+ takes after the face passes.
+__device__ __forceinline__ uint8_t* fct_classes(const StepArgs& a) { return reinterpret_cast<uint8_t*>(a.q1); }
+
 // The stage's input field (stages 1: C; 2: c1; 3: c2).
 template <int STAGE>
 __device__ __forceinline__ const double* stage_field(const StepArgs& a)
@@ -25,198 +28,247 @@ __device__ __forceinline__ const double* stage_field(const StepArgs& a)
     return STAGE == 1 ? a.C : (STAGE == 2 ? a.c1 : a.c2);
 }
 
-// The five cells of the stencil of face f (between cells f-1 and f) in upwind order, as the reference passes them
-// to _wval (sigma_baroclinic.py:277-297): v1..v5 = cells f-3 .. f+1 when the transport is >= 0, f+2 .. f-2 when it
-// is negative, with their validity `0 <= g < n and ok[g]` (periodic lines wrap).  Loading in upwind order after the
-// transport's sign is known replaces the per-value selects of a six-cell stencil (the loads wait for the transport
-// anyway: faces with Q = 0 load nothing): 1.1 % of advect_fct at 512 x 512 x 50, and fewer live registers.
-template <int ST>
-__device__ __forceinline__ void upwind5(const double* __restrict__ c, const uint8_t* __restrict__ ok, int st, int n,
-                                        bool per, int f, bool pos, double* w, bool* v)
+// Which reconstruction a face takes (sigma_baroclinic.py:204-233 `_wval`): 2 WENO5 (all five cells of its upwind
+// stencil are valid), 1 WENO3 (the middle three are), 0 the upwind cell; valid = inside the domain (or wrapped) and ok.
+// Two bits per direction of a face: bits 0-1 / 2-3 the west x-face of a cell for Q >= 0 / Q < 0, bits 4-5 / 6-7 its
+// south y-face, bits 8-9 / 10-11 (the unlimited step's uint16 classes) its bottom z-face.
+__device__ __forceinline__ unsigned stencil_class(bool a, bool b, bool c, bool d, bool e)
 {
-    const int stride = ST > 0 ? ST : st;
-    const int g0 = pos ? f - 3 : f + 2, dg = pos ? 1 : -1;
-    if (f >= 3 && f + 2 < n) {
-        const int o0 = g0 * stride, d = dg * stride;
+    return (b && c && d) ? (a && e ? 2u : 1u) : 0u;
+}
+
+// The classes of a face between cells f-1 and f from the validity of cells f-3 .. f+2.
+__device__ __forceinline__ unsigned face_class(const bool* v)
+{
+    return stencil_class(v[0], v[1], v[2], v[3], v[4]) | stencil_class(v[5], v[4], v[3], v[2], v[1]) << 2;
+}
+
+__device__ __forceinline__ unsigned line_class(const uint8_t* __restrict__ ok, int st, int n, bool per, int f)
+{
+    bool v[6];
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            w[m] = __ldg(c + (o0 + m * d));
-            v[m] = __ldg(ok + (o0 + m * d)) != 0;
-        }
-        return;
-    }
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-        int g = g0 + m * dg;
+    for (int m = 0; m < 6; ++m) {
+        int g = f - 3 + m;
         bool in = true;
         if (per) g = wrap(g, n); else in = g >= 0 && g < n;
-        w[m] = in ? __ldg(c + g * stride) : 0.0;
-        v[m] = in && __ldg(ok + (in ? g : 0) * stride) != 0;
+        v[m] = in && __ldg(ok + (in ? g : 0) * st) != 0;
     }
+    return face_class(v);
 }
 
-// One plane (t, k) of the step as pointers; element offsets below are 32-bit.
-struct FacePlane {
-    const double* __restrict__ c;     // stage field
-    const double* __restrict__ e;     // exterior on open edges (inflow, else the stage field)
-    const double* __restrict__ c0;    // C (donor flux of stage 3)
-    const double* __restrict__ e0;    // exterior of C
-    const uint8_t* __restrict__ ok;
-    const double* __restrict__ qx;
-    const double* __restrict__ qy;
-    double* sx;
-    double* sy;
-    double* tx;
-    double* ty;
-};
-
-// Flux F through x-face f of row j (WENO5 on interior faces, 0 where Q = 0; open edges upstream with the exterior
-// on inflow; closed edges 0) and, for stage 3, the donor flux FL of C through the same face
-// (sigma_baroclinic.py:277-297, 486-494).
-template <bool ZV, bool MIX, bool DONOR>
-__device__ __forceinline__ void x_face(const FacePlane& P, const Shape& s, const Flags& fl, int j, int f, double& F,
-                                       double& FL)
+// Validity of four neighbouring cells as the bytes of a word (0xff valid, 0 not): cells i .. i+3 of a row of n cells,
+// 0 outside the row (a periodic row wraps).  `row4` is the row's word when its cells may be read four at a time.
+__device__ __forceinline__ unsigned ok4(const uint8_t* __restrict__ row, int n, bool per, int i, bool words)
 {
-    const int row = j * s.nx;
-    const bool interior = fl.per_x || (f >= 1 && f <= s.nx - 1);
-    const double q = __ldg(P.qx + j * (s.nx + 1) + ((fl.per_x && f == s.nx) ? 0 : f));
-    F = 0.0;
-    FL = 0.0;
-    if (interior) {
-        if (q != 0.0) {
-            double w[5];
-            bool v[5];
-            upwind5<1>(P.c + row, P.ok + row, 1, s.nx, fl.per_x, f, q >= 0.0, w, v);
-            F = q * weno5_face<MIX>(w[0], w[1], w[2], w[3], w[4], v[0], v[1], v[2], v[3], v[4], ZV);
+    unsigned w = 0;
+    if (words && i >= 0 && i + 4 <= n) {
+        w = __ldg(reinterpret_cast<const unsigned*>(row + i));
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            int g = i + m;
+            if (per) g = wrap(g, n);
+            if (g >= 0 && g < n) w |= (unsigned)__ldg(row + g) << (8 * m);
         }
-        if (DONOR) {
-            const int ff = f == s.nx ? 0 : f;
-            const int fm = ff >= 1 ? ff - 1 : s.nx - 1;          // f >= 1 unless periodic
-            FL = q * (q >= 0 ? __ldg(P.c0 + row + fm) : __ldg(P.c0 + row + ff));
-        }
-        return;
     }
-    if (f == 0) {
-        if (fl.open_w) {
-            F = q * (q > 0.0 ? P.e[row] : P.c[row]);
-            if (DONOR) FL = q * (q > 0 ? __ldg(P.e0 + row) : __ldg(P.c0 + row));
-        }
-    } else if (fl.open_e) {
-        F = q * (q < 0.0 ? P.e[row + s.nx - 1] : P.c[row + s.nx - 1]);
-        if (DONOR) FL = q * (q < 0 ? __ldg(P.e0 + row + s.nx - 1) : __ldg(P.c0 + row + s.nx - 1));
-    }
+    return __vcmpne4(w, 0u);
 }
 
-template <bool ZV, bool MIX, bool DONOR>
-__device__ __forceinline__ void y_face(const FacePlane& P, const Shape& s, const Flags& fl, int f, int i, double& F,
-                                       double& FL)
+// The classes (see face_class) of four faces from the validity words of the cells f-3 .. f+2 of each.
+__device__ __forceinline__ unsigned class4(const unsigned* v)
 {
-    const bool interior = fl.per_y || (f >= 1 && f <= s.ny - 1);
-    const double q = __ldg(P.qy + ((fl.per_y && f == s.ny) ? 0 : f) * s.nx + i);
-    F = 0.0;
-    FL = 0.0;
-    if (interior) {
-        if (q != 0.0) {
-            double w[5];
-            bool v[5];
-            upwind5<0>(P.c + i, P.ok + i, s.nx, s.ny, fl.per_y, f, q >= 0.0, w, v);
-            F = q * weno5_face<MIX>(w[0], w[1], w[2], w[3], w[4], v[0], v[1], v[2], v[3], v[4], ZV);
-        }
-        if (DONOR) {
-            const int ff = f == s.ny ? 0 : f;
-            const int fm = ff >= 1 ? ff - 1 : s.ny - 1;
-            FL = q * (q >= 0 ? __ldg(P.c0 + fm * s.nx + i) : __ldg(P.c0 + ff * s.nx + i));
-        }
-        return;
-    }
-    if (f == 0) {
-        if (fl.open_s) {
-            F = q * (q > 0.0 ? P.e[i] : P.c[i]);
-            if (DONOR) FL = q * (q > 0 ? __ldg(P.e0 + i) : __ldg(P.c0 + i));
-        }
-    } else if (fl.open_n) {
-        const int o = (s.ny - 1) * s.nx + i;
-        F = q * (q < 0.0 ? P.e[o] : P.c[o]);
-        if (DONOR) FL = q * (q < 0 ? __ldg(P.e0 + o) : __ldg(P.c0 + o));
-    }
+    const unsigned m = v[1] & v[2] & v[3], q = v[4] & v[3] & v[2];            // the middle three, Q >= 0 / Q < 0
+    const unsigned a = m & v[0] & v[4], b = q & v[5] & v[1];                  // all five
+    return (a & 0x02020202u) | (m & ~a & 0x01010101u) | (b & 0x08080808u) | (q & ~b & 0x04040404u);
 }
 
-// Store the stage's quantity of one face (S, T: the face arrays of this plane).  Stages 3 and 4 read the face's F0
-// and F1 here, after the face computation: holding them across the WENO chains cost registers, and at the face
-// passes' 32-register budget the spills outweighed the overlap (2.2 % of advect_fct at 512 x 512 x 50).
-template <int STAGE>
-__device__ __forceinline__ void put_face(double* S, double* T, int fo, double F, double FL)
-{
-    if (STAGE == 1) {
-        S[fo] = F;
-    } else if (STAGE == 2) {
-        T[fo] = F;
-    } else if (STAGE == 3) {
-        S[fo] = (div6_exact(S[fo] + T[fo]) + div3_exact(2.0 * F)) - FL;
-    } else {                     // the unlimited step: S <- the RK3 flux F_H = (F0 + F1)/6 + 2 F2/3
-        S[fo] = div6_exact(S[fo] + T[fo]) + div3_exact(2.0 * F);
-    }
-}
-
-// Face pass of stage STAGE for cell (t, k, j, i); blocks are 32 x TJR cells of one (t, k) plane, planes k-major (the
-// tracers of a layer in a row share the layer's transports in L2).
-template <int STAGE, bool ZV, bool MIX>
-__device__ __forceinline__ void faces_body(const StepArgs& a, int t, int k, int i, int j)
+// Class pass: works out the classes of every cell's two faces once for the three face passes and every tracer (they
+// depend on ok alone), one byte per cell; the face passes used to load and test five ok bytes per stencil.  A thread
+// takes four neighbouring cells, their validity in the bytes of a word; where nx is a multiple of four and ok starts
+// on a word, rows are read and written by words.
+__device__ __forceinline__ void class_body(const StepArgs& a, int k, int i, int j)
 {
     const Shape s = a.s;
     const Flags fl(a.flags);
     if (i >= s.nx || j >= s.ny) return;
-    const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx, p = t * s.n + k;
-    const i64 pc = plane_at(p, pl), pu = plane_at(p, xpl), pv = plane_at(p, ypl);
-    FacePlane P;
-    P.c = stage_field<STAGE>(a) + pc;
-    P.e = a.inflow ? a.inflow + pc : P.c;
-    P.c0 = a.C + pc;
-    P.e0 = a.inflow ? a.inflow + pc : P.c0;
-    P.ok = a.ok + plane_at(k, pl);
-    P.qx = a.Qx + plane_at(k, xpl);
-    P.qy = a.Qy + plane_at(k, ypl);
-    P.sx = a.Sx + pu;
-    P.sy = a.Sy + pv;
-    P.tx = a.Tx + pu;
-    P.ty = a.Ty + pv;
-    const int fxo = j * (s.nx + 1) + i, fyo = j * s.nx + i;
-    const bool last_x = i == s.nx - 1, last_y = j == s.ny - 1;
-    double fw, lw, fs, ls, le = 0.0, ln = 0.0;
-    x_face<ZV, MIX, STAGE == 3>(P, s, fl, j, i, fw, lw);
-    y_face<ZV, MIX, STAGE == 3>(P, s, fl, j, i, fs, ls);
-    put_face<STAGE>(P.sx, P.tx, fxo, fw, lw);
-    put_face<STAGE>(P.sy, P.ty, fyo, fs, ls);
-    if (last_x) {
-        double fe;
-        x_face<ZV, MIX, STAGE == 3>(P, s, fl, j, s.nx, fe, le);
-        put_face<STAGE>(P.sx, P.tx, fxo + 1, fe, le);
+    const int pl = s.ny * s.nx;
+    const uint8_t* ok = a.ok + plane_at(k, pl);
+    const bool words = (s.nx & 3) == 0 && (reinterpret_cast<uintptr_t>(ok) & 3) == 0;
+    const uint8_t* row = ok + j * s.nx;
+    const unsigned w0 = ok4(row, s.nx, fl.per_x, i - 4, words), w1 = ok4(row, s.nx, fl.per_x, i, words),
+                   w2 = ok4(row, s.nx, fl.per_x, i + 4, words);
+    unsigned v[6];
+    v[0] = __funnelshift_r(w0, w1, 8);                                        // cells i-3 .. i
+    v[1] = __funnelshift_r(w0, w1, 16);
+    v[2] = __funnelshift_r(w0, w1, 24);
+    v[3] = w1;
+    v[4] = __funnelshift_r(w1, w2, 8);
+    v[5] = __funnelshift_r(w1, w2, 16);
+    unsigned c = class4(v);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+        int g = j - 3 + m;
+        if (fl.per_y) g = wrap(g, s.ny);
+        v[m] = m == 3 ? w1 : (g >= 0 && g < s.ny ? ok4(ok + g * s.nx, s.nx, false, i, words) : 0u);
     }
-    if (last_y) {
-        double fn;
-        y_face<ZV, MIX, STAGE == 3>(P, s, fl, s.ny, i, fn, ln);
-        put_face<STAGE>(P.sy, P.ty, fyo + s.nx, fn, ln);
+    c |= class4(v) << 4;
+    uint8_t* out = fct_classes(a) + plane_at(k, pl) + (j * s.nx + i);
+    if (words) {
+        *reinterpret_cast<unsigned*>(out) = c;
+        return;
     }
-    if (STAGE == 3) {
-        // c_L = safe(q0 - dt div F_L, V1) of this cell (sigma_baroclinic.py:509-511): the donor fluxes of its east
-        // and north faces are recomputed here (they are its neighbours' west and south faces), so F_L is never
-        // stored and no separate cell pass runs
-        // faces i + 1 <= nx - 1 and j + 1 <= ny - 1 are interior on any axis (periodic or not)
-        const double c0 = __ldg(P.c0 + fyo);
-        if (!last_x) {
-            const double q = __ldg(P.qx + fxo + 1);
-            le = q * (q >= 0 ? c0 : __ldg(P.c0 + fyo + 1));
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        if (i + m < s.nx) out[m] = (uint8_t)(c >> (8 * m));
+}
+
+// Face value of an interior face from its class (the face lies between cells f-1 and f of a line of n cells `st`
+// apart; o: the offset of cell f).  The cells are loaded in upwind order v1..v5, as the reference passes them to
+// _wval: cells f-3 .. f+1 for Q >= 0, f+2 .. f-2 for Q < 0.  A class only counts cells inside the domain, so only a
+// periodic line's stencil needs to wrap, at its ends (INNER: the face is at least three cells from them).
+template <bool ZV, bool MIX, bool INNER>
+__device__ __forceinline__ double face_value(const double* __restrict__ c, int o, int st, int n, bool per, int f,
+                                             bool pos, unsigned cls)
+{
+    const int d = pos ? st : -st;
+    int o3 = pos ? o - st : o, o1 = o3 - 2 * d, o2 = o3 - d, o4 = o3 + d, o5 = o4 + d;
+    if (!INNER && per && (f < 3 || f + 2 >= n)) {
+        const int ln = n * st, l0 = o - f * st;           // offsets of this line run from l0 to l0 + ln
+        auto in = [&](int x) { x -= l0; return l0 + (((unsigned)x < (unsigned)ln) ? x : wrap(x, ln)); };
+        o1 = in(o1); o2 = in(o2); o3 = in(o3); o4 = in(o4); o5 = in(o5);
+    }
+    if (cls == 2u) return weno5_any<ZV, MIX>(__ldg(c + o1), __ldg(c + o2), __ldg(c + o3), __ldg(c + o4), __ldg(c + o5));
+    const double v3 = __ldg(c + o3);
+    if (cls == 0u) return v3;
+    return weno3_any<MIX>(__ldg(c + o2), v3, __ldg(c + o4));
+}
+
+// The stage's quantity of one face (S, T: the face arrays of this plane), read back for stages 3 and 4 here, after
+// the face computation: holding them across the WENO chains cost registers, and at the face passes' 32-register
+// budget the spills outweighed the overlap (2.2 % of advect_fct at 512 x 512 x 50).  The thirds and sixths
+// of zeros (land and closed faces, still tracers) take their short form: through two divisions each they cost stage 3
+// half as many instructions again.
+template <int STAGE>
+__device__ __forceinline__ double staged_flux(const double* S, const double* T, int fo, double F, double FL)
+{
+    if (STAGE <= 2) return F;
+    const double H = div6_exact(S[fo] + T[fo]) + div3_exact(2.0 * F);
+    return STAGE == 3 ? H - FL : H;               // 4, the unlimited step: the RK3 flux F_H = (F0 + F1)/6 + 2 F2/3
+}
+
+// Flux through a domain-edge face (west / south: SIDE 1, inflow for q > 0; east / north: -1): upstream on an open
+// edge with the exterior on inflow, 0 on a closed one (sigma_baroclinic.py:283-297); c, e: the edge cell's value and
+// its exterior's.
+template <int SIDE>
+__device__ __forceinline__ double edge_flux(bool open, double q, double c, double e)
+{
+    return open ? q * ((SIDE > 0 ? q > 0.0 : q < 0.0) ? e : c) : 0.0;
+}
+
+// Face pass of stage STAGE for cell (k, j, i) of tracers t0 .. t1-1.  Flux through the cell's west x-face and south
+// y-face: WENO5 on interior faces, 0 where Q = 0; stage 3 also the donor flux F_L of C (sigma_baroclinic.py:277-297,
+// 486-494).  The last column / row adds the east / north domain face; on a periodic axis that face is face 0, which
+// the first column / row stores twice.  INNER: the cell is at least three cells from every domain edge, where none of
+// that arises.
+template <int STAGE, bool ZV, bool MIX, bool INNER>
+__device__ __forceinline__ void faces_cell(const StepArgs& a, int t0, int t1, int k, int i, int j)
+{
+    const Shape s = a.s;
+    const Flags fl(a.flags);
+    const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx;
+    const int o = j * s.nx + i, ox = o + j;
+    const double* __restrict__ qx = a.Qx + plane_at(k, xpl);
+    const double* __restrict__ qy = a.Qy + plane_at(k, ypl);
+    const unsigned cls = __ldg(fct_classes(a) + plane_at(k, pl) + o);
+    const double qw = __ldg(qx + ox), qs = __ldg(qy + o);
+    const bool per_x = !INNER && fl.per_x, per_y = !INNER && fl.per_y;
+    const bool last_x = !INNER && i == s.nx - 1, last_y = !INNER && j == s.ny - 1;
+#pragma unroll 1
+    for (int t = t0; t < t1; ++t) {
+        const int p = t * s.n + k;
+        const i64 pc = plane_at(p, pl), pu = plane_at(p, xpl), pv = plane_at(p, ypl);
+        const double* __restrict__ c = stage_field<STAGE>(a) + pc;
+        const double* __restrict__ c0 = a.C + pc;                    // the donor flux of stage 3
+        double* sx = (STAGE == 2 ? a.Tx : a.Sx) + pu;
+        double* sy = (STAGE == 2 ? a.Ty : a.Sy) + pv;
+        const double* tx = a.Tx + pu;
+        const double* ty = a.Ty + pv;
+        double fw = 0.0, lw = 0.0, fs = 0.0, ls = 0.0;
+        // west x-face
+        if (INNER || per_x || i >= 1) {
+            if (qw != 0.0) {
+                const bool pos = qw >= 0.0;
+                fw = qw * face_value<ZV, MIX, INNER>(c, o, 1, s.nx, per_x, i, pos, (pos ? cls : cls >> 2) & 3u);
+            }
+            if (STAGE == 3) lw = qw * __ldg(c0 + (qw >= 0 ? (INNER || i >= 1 ? o - 1 : o + s.nx - 1) : o));
+        } else {
+            fw = edge_flux<1>(fl.open_w, qw, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+            if (STAGE == 3) lw = edge_flux<1>(fl.open_w, qw, c0[o], a.inflow ? a.inflow[pc + o] : c0[o]);
         }
-        if (!last_y) {
-            const double q = __ldg(P.qy + fyo + s.nx);
-            ln = q * (q >= 0 ? c0 : __ldg(P.c0 + fyo + s.nx));
+        const double aw = staged_flux<STAGE>(sx, tx, ox, fw, lw);
+        sx[ox] = aw;
+        if (per_x && i == 0) sx[ox + s.nx] = aw;
+        // south y-face
+        if (INNER || per_y || j >= 1) {
+            if (qs != 0.0) {
+                const bool pos = qs >= 0.0;
+                fs = qs * face_value<ZV, MIX, INNER>(c, o, s.nx, s.ny, per_y, j, pos, (pos ? cls >> 4 : cls >> 6) & 3u);
+            }
+            if (STAGE == 3) ls = qs * __ldg(c0 + (qs >= 0 ? (INNER || j >= 1 ? o - s.nx : o + pl - s.nx) : o));
+        } else {
+            fs = edge_flux<1>(fl.open_s, qs, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+            if (STAGE == 3) ls = edge_flux<1>(fl.open_s, qs, c0[o], a.inflow ? a.inflow[pc + o] : c0[o]);
         }
-        const double dl = le - lw + ln - ls;
-        const i64 g = plane_at(k, pl) + fyo;
-        const double v0 = __ldg(a.V0 + g), v1 = __ldg(a.V1 + g);
-        const double q0 = v0 * c0;
-        const double q = 0.0 * q0 + 1.0 * (q0 - a.dt * dl);
-        a.q1[pc + fyo] = v1 > 0 ? q / v1 : c0;
+        const double as = staged_flux<STAGE>(sy, ty, o, fs, ls);
+        sy[o] = as;
+        if (per_y && j == 0) sy[o + pl] = as;
+        // east / north domain faces of a closed or open axis
+        double le = 0.0, ln = 0.0;
+        if (last_x && !per_x) {
+            const double q = __ldg(qx + (ox + 1));
+            const double fe = edge_flux<-1>(fl.open_e, q, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+            if (STAGE == 3) le = edge_flux<-1>(fl.open_e, q, c0[o], a.inflow ? a.inflow[pc + o] : c0[o]);
+            sx[ox + 1] = staged_flux<STAGE>(sx, tx, ox + 1, fe, le);
+        }
+        if (last_y && !per_y) {
+            const double q = __ldg(qy + (o + s.nx));
+            const double fn = edge_flux<-1>(fl.open_n, q, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+            if (STAGE == 3) ln = edge_flux<-1>(fl.open_n, q, c0[o], a.inflow ? a.inflow[pc + o] : c0[o]);
+            sy[o + s.nx] = staged_flux<STAGE>(sy, ty, o + s.nx, fn, ln);
+        }
+        if (STAGE == 3) {
+            // c_L = safe(q0 - dt div F_L, V1) of this cell (sigma_baroclinic.py:509-511): the donor fluxes of its
+            // east and north faces are recomputed here (they are its neighbours' west and south faces), so F_L is
+            // never stored and no separate cell pass runs.  c_L goes over c1, which no pass after stage 2 reads.
+            const double cc = __ldg(c0 + o);
+            if (!last_x || per_x) {
+                const double q = __ldg(qx + (last_x ? ox + 1 - s.nx : ox + 1));
+                le = q * (q >= 0 ? cc : __ldg(c0 + (last_x ? o + 1 - s.nx : o + 1)));
+            }
+            if (!last_y || per_y) {
+                const double q = __ldg(qy + (last_y ? i : o + s.nx));
+                ln = q * (q >= 0 ? cc : __ldg(c0 + (last_y ? i : o + s.nx)));
+            }
+            const double dl = le - lw + ln - ls;
+            const i64 g = plane_at(k, pl);
+            const double v0 = __ldg(a.V0 + g + o), v1 = __ldg(a.V1 + g + o);
+            const double q0 = v0 * cc;
+            const double q = 0.0 * q0 + 1.0 * (q0 - a.dt * dl);
+            (a.c1 + pc)[o] = v1 > 0 ? q / v1 : cc;
+        }
+    }
+}
+
+// The cell's pass, with the domain-edge cases left out where the block of cells (TI x TJR from (i0, j0)) is at least
+// three cells from every edge (85 % of the blocks at 512 x 512).
+template <int STAGE, bool ZV, bool MIX, int TJR>
+__device__ __forceinline__ void faces_body(const StepArgs& a, int t0, int t1, int k, int i0, int j0)
+{
+    const int i = i0 + threadIdx.x % TI, j = j0 + threadIdx.x / TI;
+    if (i0 >= 3 && j0 >= 3 && i0 + TI + 2 <= a.s.nx && j0 + TJR + 2 <= a.s.ny) {
+        faces_cell<STAGE, ZV, MIX, true>(a, t0, t1, k, i, j);
+    } else if (i < a.s.nx && j < a.s.ny) {
+        faces_cell<STAGE, ZV, MIX, false>(a, t0, t1, k, i, j);
     }
 }
 
@@ -241,12 +293,26 @@ __device__ __forceinline__ void faces_body(const StepArgs& a, int t, int k, int 
 #endif
 #define FACES12_BOUNDS(n) __launch_bounds__(n, (MIX ? POCEAN_FACES12_MINB_MIX : POCEAN_FACES12_MINB) * 256 / (n))
 #define FACES3_BOUNDS(n) __launch_bounds__(n, (MIX ? POCEAN_FACES3_MINB_MIX : POCEAN_FACES3_MINB) * 256 / (n))
+// The layer and the tracers t0 .. t1-1 of a single-domain face CTA: every tracer of layer blockIdx.z, or, where those
+// CTAs would leave the chip idle (StepArgs::per_plane), the one tracer of plane blockIdx.z.
+__device__ __forceinline__ void split_tracers(const StepArgs& a, int& k, int& t0, int& t1)
+{
+    if (a.per_plane) {
+        split_plane(a.k0 * a.s.nt + blockIdx.z, a.s.nt, a.tdiv, k, t0);
+        t1 = t0 + 1;
+    } else {
+        k = a.k0 + blockIdx.z;
+        t0 = 0;
+        t1 = a.s.nt;
+    }
+}
+
 template <int STAGE, bool ZV, bool MIX, int TJR>
 __device__ __forceinline__ void faces_plane(const StepArgs& a)
 {
-    int k, t;
-    split_plane(a.k0 * a.s.nt + blockIdx.z, a.s.nt, a.tdiv, k, t);
-    faces_body<STAGE, ZV, MIX>(a, t, k, blockIdx.x * TI + threadIdx.x % TI, blockIdx.y * TJR + threadIdx.x / TI);
+    int k, t0, t1;
+    split_tracers(a, k, t0, t1);
+    faces_body<STAGE, ZV, MIX, TJR>(a, t0, t1, k, blockIdx.x * TI, blockIdx.y * TJR);
 }
 
 template <int STAGE, bool ZV, bool MIX, int TJR>
@@ -261,18 +327,23 @@ __global__ void FACES3_BOUNDS(TI * TJR) fct_faces3_kernel(StepArgs a)
     faces_plane<3, ZV, MIX, TJR>(a);
 }
 
-// Where a batched CTA works (domain d owns CTAs off[d] .. off[d+1]-1): its domain d, tracer t and layer k, and its
-// 32 x TJR tile (bx, by).  The first thread of
-// the CTA works it out (a binary search over the domains' CTA offsets and two integer divisions, the same for every
-// thread of the CTA) and shares it, with the domain's argument block, through shared memory: done by every thread,
-// that set-up cost the batched cell passes as many instructions again as their own work.
+template <int TJR>
+__global__ void __launch_bounds__(TI * TJR) fct_class_kernel(StepArgs a)
+{
+    class_body(a, a.k0 + blockIdx.z, 4 * (blockIdx.x * TI + threadIdx.x % TI), blockIdx.y * TJR + threadIdx.x / TI);
+}
+
+// Where a batched CTA works (domain d owns CTAs off[d] .. off[d+1]-1): its domain d, its layer k (and
+// tracer t) and its 32 x TJR tile (bx, by).  The first thread of the CTA works it out (a binary search over the domains' CTA offsets and two integer
+// divisions, the same for every thread of the CTA) and shares it, with the domain's argument block, through shared
+// memory: done by every thread, that set-up cost the batched cell passes as many instructions again as their own work.
 struct BlockTile {
     int d, t, k, bx, by;
 };
 
 // The CTA's tile (bt) and its domain's argument block (sh), both in shared memory.  PLANES: the CTA's index counts
-// 32 x TJR tiles of the (t, k) planes (k-major: the stage passes); else tiles of the layers (t = 0: the coefficient
-// and final passes).  Call before any thread returns: it contains block barriers.
+// tiles of the (t, k) planes (k-major: the cell passes); else tiles of the layers (t = 0).  Call before any thread
+// returns: it contains block barriers.
 template <bool PLANES, int TJR>
 __device__ __forceinline__ const StepArgs& block_tile(const BatchDomain* __restrict__ doms, const int* __restrict__ off,
                                                       int ndom, BlockTile& bt, StepArgs& sh)
@@ -303,8 +374,8 @@ __device__ __forceinline__ void faces_batched_body(const BatchDomain* __restrict
 {
     __shared__ BlockTile bt;
     __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<true, TJR>(doms, off, ndom, bt, sh);
-    faces_body<STAGE, ZV, MIX>(a, bt.t, bt.k, bt.bx * TI + threadIdx.x % TI, bt.by * TJR + threadIdx.x / TI);
+    const StepArgs& a = block_tile<false, TJR>(doms, off, ndom, bt, sh);
+    faces_body<STAGE, ZV, MIX, TJR>(a, 0, a.s.nt, bt.k, bt.bx * TI, bt.by * TJR);
 }
 
 template <int STAGE, bool ZV, bool MIX, int TJR>
@@ -319,6 +390,15 @@ __global__ void FACES3_BOUNDS(TI * TJR) fct_faces3_batched(const BatchDomain* __
                                                            const int* __restrict__ off, int ndom)
 {
     faces_batched_body<3, ZV, MIX, TJR>(doms, off, ndom);
+}
+
+__global__ void __launch_bounds__(NTHREADS / 4) fct_class_batched(const BatchDomain* __restrict__ doms,
+                                                              const int* __restrict__ off, int ndom)
+{
+    __shared__ BlockTile bt;
+    __shared__ StepArgs sh;
+    const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
+    class_body(a, bt.k, bt.bx * TI + 4 * (threadIdx.x % (TI / 4)), bt.by * TJ + threadIdx.x / (TI / 4));
 }
 
 // Cell pass of stage STAGE = 1, 2 (sigma_baroclinic.py:452-468 `_fct_stage`); stage 3 has none (its face pass

@@ -179,7 +179,7 @@ class Server:
                 for j in step_set:
                     for s in range(k):
                         sequential_step([j.dom], j.flip ^ (s & 1), mixed=self.mixed, stream=stream.cuda_stream)
-                launches += k * sum(7 + (j.nt >= 2) + (j.nt % 2) + 1 for j in step_set)
+                launches += k * sum(8 + (j.nt >= 2) + (j.nt % 2) + 1 for j in step_set)
             iters += 1
             occupancy.append(len(step_set))
             done = []
@@ -241,7 +241,7 @@ class Server:
 
     def _launches(self, active) -> int:
         if self.remap_nf == 2:
-            return 7 + any(j.nt >= 2 for j in active) + any(j.nt % 2 for j in active) + 1
+            return 8 + any(j.nt >= 2 for j in active) + any(j.nt % 2 for j in active) + 1
         return 9
 
     def _retire(self, j: Job, stream) -> None:
