@@ -17,6 +17,7 @@ struct pocean_batch {
     int tile_rows;                     // rows of the 32-wide tiles of the stage passes
     int nmax;                          // deepest column of the batch
     bool zv;                           // WENO5-Z (else JS) for every domain
+    bool segments;                     // the remap's form (remap_batch_segments)
     BatchDomain* dev_doms;             // 2 * ndom descriptors: parity 0 then parity 1
     int* dev_off;                      // BP_COUNT * (ndom + 1) offsets
     std::vector<int> host_off;
@@ -47,6 +48,11 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     std::vector<int> off((size_t)BP_COUNT * (ndom + 1), 0);
     const bool zv = !(domains[0].flags & POCEAN_WENO_JS);
     int nmax = 1;
+    for (int d = 0; d < ndom; ++d) nmax = domains[d].nz > nmax ? domains[d].nz : nmax;
+    long long all_columns = 0;
+    for (int d = 0; d < ndom; ++d) all_columns += (long long)domains[d].ny * domains[d].nx * domains[d].nt;
+    const bool segments = remap_batch_segments(all_columns, nmax);
+    const int columns = remap_batched_columns(segments);
     long long tot[BP_COUNT] = {};
     for (int d = 0; d < ndom; ++d) {
         const pocean_domain& D = domains[d];
@@ -66,7 +72,6 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
         const size_t need = pocean_advect_fct_workspace_bytes(D.nt, D.nz, D.ny, D.nx);
         if (!D.workspace || D.workspace_bytes < need || ((uintptr_t)D.workspace & 255))
             return pocean_fail(POCEAN_EWORKSPACE, "%s: domain %d: workspace of %zu bytes needed", fn, d, need);
-        nmax = D.nz > nmax ? D.nz : nmax;
         for (int parity = 0; parity < 2; ++parity) {
             BatchDomain& B = host[(size_t)parity * ndom + d];
             std::memset(&B, 0, sizeof(B));
@@ -84,8 +89,8 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
             int pc, lc, tc;
             fct_batched_ctas(B.a.s, tile_rows, pc, lc, tc);
             if (parity == 0) {
-                const long long cb = ((long long)D.ny * D.nx + 127) / 128;
-                const long long n_pass[BP_COUNT] = {pc, lc, tc, cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt, cb * D.nt};
+                const long long cb = ((long long)D.ny * D.nx + columns - 1) / columns;
+                const long long n_pass[BP_COUNT] = {pc, lc, tc, cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt};
                 for (int q = 0; q < BP_COUNT; ++q) {
                     off[(size_t)q * (ndom + 1) + d] = (int)tot[q];
                     tot[q] += n_pass[q];
@@ -101,6 +106,7 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     b->tile_rows = tile_rows;
     b->nmax = nmax;
     b->zv = zv;
+    b->segments = segments;
     b->dev_doms = (BatchDomain*)device_buf;
     b->dev_off = (int*)((char*)device_buf + (((size_t)2 * ndom * sizeof(BatchDomain) + 255) & ~(size_t)255));
     b->host_off = off;
@@ -128,7 +134,9 @@ extern "C" int pocean_batch_step(const pocean_batch* b, int parity, int remap_nf
     cudaStream_t st = (cudaStream_t)stream;
     const BatchDomain* doms = b->dev_doms + (size_t)parity * b->ndom;
     fct_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, b->zv, mixed != 0, b->tile_rows, st);
-    remap_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, remap_nf, b->nmax, st);
+    const cudaError_t e = remap_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, remap_nf, b->nmax,
+                                               b->segments, st);
+    if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
     return pocean_check_launch(fn);
 }
 

@@ -72,7 +72,7 @@ enum BatchPass {
     BP_PTILE = 0,       // tile_rows tiles of the (tracer, layer) planes: cell passes
     BP_LTILE,           // tile_rows tiles of the layers: face passes
     BP_TILE,            // 8-row tiles of the layers: class, coefficient and final passes
-    BP_RPAIR, BP_RREM, BP_RALL, BP_RGEN,
+    BP_RPAIR, BP_RREM, BP_RALL,     // column groups x field pairs, odd fields, all fields: remap
     BP_COUNT
 };
 
@@ -109,7 +109,9 @@ void carve_fct_workspace(StepArgs& a, void* workspace);
 void fct_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, bool zv,
                         bool mixed, int tile_rows, cudaStream_t st);
 void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& layer_ctas, int& tile_ctas);
-void remap_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int nf_mode,
-                          int nmax, cudaStream_t st);
+bool remap_batch_segments(long long columns, int nmax);
+int remap_batched_columns(bool segments);
+cudaError_t remap_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int nf_mode,
+                                 int nmax, bool segments, cudaStream_t st);
 
 }  // namespace po

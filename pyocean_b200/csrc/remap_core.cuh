@@ -166,12 +166,17 @@ PO_HD H4Weights h4_weights(double h0, double h1, double h2, double h3)
     return w;
 }
 
-PO_HD double h4_edge(const H4Weights& w, double u0, double u1, double u2, double u3)
+PO_HD double h4_numerator(const H4Weights& w, double u0, double u1, double u2, double u3)
 {
     const double et1 = w.w1 * u1 + w.w2 * u2;
     const double et2 = w.g2 * (u1 - u0);
     const double et3 = w.g3 * (u2 - u3);
-    return (et1 + (et2 + et3)) / w.den;
+    return et1 + (et2 + et3);
+}
+
+PO_HD double h4_edge(const H4Weights& w, double u0, double u1, double u2, double u3)
+{
+    return h4_numerator(w, u0, u1, u2, u3) / w.den;
 }
 
 // The limiter steps below (bound_slope, bound_edge, check_pair, ppm_coef) are written without branches: each
