@@ -9,16 +9,17 @@
 //
 // Mapping: one thread per face column (j, f) or per cell column / cell-layer; consecutive threads take consecutive
 // i (or f), so every per-layer access of a warp is one contiguous segment.  The Newton iteration of the PPM
-// transport stops when every face has converged (the reference's global test): iteration i is one launch that
-// first reads how many faces iteration i-1 left unconverged and returns at once when none, so max_iter launches are
-// enqueued without a host round trip.  The outflow limiter's passes end on a global test too; it is rare (nothing
-// to limit in the common case) and synchronises once per pass.
+// transport stops when every face has converged (the reference's global test); columns of up to 80 layers iterate inside
+// one CTA (ppm_newton_kernel), deeper ones in one launch per iteration, which first reads how many faces the one before
+// left unconverged and returns at once when none.  The outflow limiter's passes end on a global test too; it is rare
+// (nothing to limit in the common case) and synchronises once per pass.
 #include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstring>
 
 #include "common.cuh"
+#include "exactdiv.cuh"
 
 namespace po {
 namespace pr {
@@ -104,49 +105,48 @@ struct Thick {
     const uint8_t* __restrict__ act;
     int pc;
     int nx;
-    __device__ __forceinline__ double at(int k, int j, int i) const
-    {
-        return __ldg(act + (j * nx + i)) ? nan_to_num(__ldg(h + (k * pc + j * nx + i))) : 0.0;
-    }
-    __device__ __forceinline__ double m(int j, int i) const { return __ldg(act + (j * nx + i)) ? 1.0 : 0.0; }
 };
 
-// The limited slope of cell i (first loop of _ppm_edges_kernel).
-__device__ __forceinline__ double ppm_slope(const Thick& T, int k, int j, int i)
+// ale.py:582-626: edge values of the cells of row j, layer k.  A warp takes 32 neighbouring cells of a row and writes the
+// 30 inside: each lane reads its own cell and works out its limited slope once, and its neighbours' thicknesses, masks
+// and slopes come by shuffles.  With each thread forming the slopes of its cell and both neighbours it was bound by
+// instructions (733 per warp) and took 180 us at 384 x 384 x 50, now 87.
+constexpr int EDGE_WARPS = 4;
+__global__ void __launch_bounds__(32 * EDGE_WARPS) ppm_edges_kernel(Thick T, int n, int ny, double h_min,
+                                                                    double* __restrict__ h_w, double* __restrict__ h_e)
 {
-    const int nx = T.nx;
-    const double m = T.m(j, i);
-    const double mw = i > 0 ? T.m(j, i - 1) : 0.0;
-    const double me = i < nx - 1 ? T.m(j, i + 1) : 0.0;
-    const double hc = T.at(k, j, i);
-    const double hm1 = i > 0 ? mw * T.at(k, j, i - 1) + (1.0 - mw) * hc : hc;
-    const double hp1 = i < nx - 1 ? me * T.at(k, j, i + 1) + (1.0 - me) * hc : hc;
+    const int nx = T.nx, lane = threadIdx.x & 31;
+    const int i = (blockIdx.x * EDGE_WARPS + (threadIdx.x >> 5)) * 30 - 1 + lane;
+    const int j = blockIdx.y, k = blockIdx.z;
+    constexpr unsigned all = 0xffffffffu;
+    // thickness and mask of the cells i - 1, i, i + 1 (no cell outside the row)
+    auto load = [&](int c, double& h, double& m) {
+        const bool act = c >= 0 && c < nx && __ldg(T.act + (j * nx + c)) != 0;
+        m = act ? 1.0 : 0.0;
+        h = act ? nan_to_num(__ldg(T.h + (k * T.pc + j * nx + c))) : 0.0;
+    };
+    double hc, m, hw_, mw, he_, me;
+    load(i, hc, m);
+    hw_ = __shfl_up_sync(all, hc, 1);
+    mw = __shfl_up_sync(all, m, 1);
+    he_ = __shfl_down_sync(all, hc, 1);
+    me = __shfl_down_sync(all, m, 1);
+    if (lane == 0) load(i - 1, hw_, mw);
+    if (lane == 31) load(i + 1, he_, me);
+    const double hm1 = i > 0 ? mw * hw_ + (1.0 - mw) * hc : hc;
+    const double hp1 = i < nx - 1 ? me * he_ + (1.0 - me) * hc : hc;
+    // the limited slope (first loop of _ppm_edges_kernel)
     double s = 0.5 * (hp1 - hm1);
     const double dmx = pmax(pmax(hp1, hm1), hc) - hc;
     const double dmn = hc - pmin(pmin(hp1, hm1), hc);
-    const double a = pmin(fabs(s), 2.0 * pmin(dmx, dmn));
-    s = s > 0.0 ? a : (s < 0.0 ? -a : 0.0);
-    return mw * me * m > 0.0 ? s : 0.0;
-}
-
-// ale.py:582-626: edge values of cell (k, j, i); the neighbours' slopes are recomputed from h, not stored.
-__global__ void __launch_bounds__(128) ppm_edges_kernel(Thick T, int n, int ny, double h_min, double* __restrict__ h_w,
-                                                        double* __restrict__ h_e)
-{
-    const int nx = T.nx;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= nx) return;
-    const double mw = i > 0 ? T.m(j, i - 1) : 0.0;
-    const double me = i < nx - 1 ? T.m(j, i + 1) : 0.0;
-    const double hc = T.at(k, j, i);
-    const double hm1 = i > 0 ? mw * T.at(k, j, i - 1) + (1.0 - mw) * hc : hc;
-    const double hp1 = i < nx - 1 ? me * T.at(k, j, i + 1) + (1.0 - me) * hc : hc;
-    const double sc_ = ppm_slope(T, k, j, i);
-    const double sw = i > 0 ? ppm_slope(T, k, j, i - 1) : 0.0;
-    const double se = i < nx - 1 ? ppm_slope(T, k, j, i + 1) : 0.0;
-    const double hw = 0.5 * (hm1 + hc) + (sw - sc_) / 6.0;
-    const double he = 0.5 * (hp1 + hc) + (sc_ - se) / 6.0;
+    const double lim = pmin(fabs(s), 2.0 * pmin(dmx, dmn));
+    s = s > 0.0 ? lim : (s < 0.0 ? -lim : 0.0);
+    s = mw * me * m > 0.0 ? s : 0.0;
+    const double su = __shfl_up_sync(all, s, 1), sd = __shfl_down_sync(all, s, 1);
+    if (lane == 0 || lane == 31 || i >= nx) return;
+    const double sw = i > 0 ? su : 0.0, se = i < nx - 1 ? sd : 0.0;
+    const double hw = 0.5 * (hm1 + hc) + div6_exact(sw - s);
+    const double he = 0.5 * (hp1 + hc) + div6_exact(s - se);
     const double curv = 3.0 * ((hw + he) - 2.0 * hc);
     const double dh = he - hw;
     const bool inside = curv > 0.0 && fabs(dh) < curv;
@@ -368,6 +368,291 @@ __global__ void PPM_BOUNDS ppm_final_kernel(PPMArgs a, double* __restrict__ out)
     const double den = tot > 0.0 ? tot : 1.0;
     const double* qs = use_e ? a.q_e : a.q_w;
     for (int k = 0; k < a.n; ++k) out[k * pf + o] = out[k * pf + o] + R * __ldg(qs + k * pf + o) / den;
+}
+
+// One face's whole correction by the general passes' arithmetic, read from memory layer by layer: the faces of
+// ppm_newton_kernel outside the ranges of its short quotients (velocities or widths that are not finite, or whose
+// exponents are beyond +-250).
+static __device__ __noinline__ void ppm_face_general(const PPMArgs& a, int o, int steps, int max_iter, bool mark,
+                                                     double* __restrict__ out)
+{
+    const int nf = a.nx + 1, pf = a.ny * nf, j = o / nf, f = o - j * nf;
+    const FaceCells fc = face_cells(a, j, f);
+    const bool open = fc.aw && fc.ae;
+    const double limw = 0.5 * fc.dxw / a.dt, lime = 0.5 * fc.dxe / a.dt, q = __ldg(a.Q_bt + o), L_f = __ldg(a.L + o);
+    double mnw = INFINITY, mxe = -INFINITY;
+    for (int k = 0; k < a.n; ++k) {
+        const double u = __ldg(a.ut + k * pf + o);
+        mnw = pmin(mnw, limw - u);
+        mxe = pmax(mxe, -(lime + u));
+    }
+    double hi = pmax(pmin(limw, mnw), 0.0), lo = pmin(pmax(-lime, mxe), 0.0), du = 0.0, s, ds;
+    column_flux(a, j, f, 0.0, false, s, ds);
+    double err = s - q;
+    for (int it = 0; it < steps; ++it) {
+        const double d = du;
+        if (err > 0.0) hi = d;
+        if (err < 0.0) lo = d;
+        const double step = ds > 0.0 ? -err / ds : 0.0;
+        double nw = d + step;
+        if (step > 0.0 && nw >= hi) nw = 0.5 * (d + hi);
+        if (step < 0.0 && nw <= lo) nw = 0.5 * (d + lo);
+        du = nw;
+        column_flux(a, j, f, du, true, s, ds);
+        err = s - q;
+        if (mark && fabs(err) > 1e-12 * pmax(fabs(q), 1.0)) a.unconverged[it] = 1;
+    }
+    double te = 0.0, tw = 0.0;
+    s = 0.0;
+    for (int k = 0; k < a.n; ++k) {
+        double F = 0.0, dF;
+        if (open) face_flux(a, fc, k, o, __ldg(a.ut + k * pf + o) + du, L_f, F, dF);
+        out[k * pf + o] = F;
+        s += F;
+        te += __ldg(a.q_e + k * pf + o);
+        tw += __ldg(a.q_w + k * pf + o);
+    }
+    if (!open) return;
+    const double R = q - s;
+    bool use_e = R >= 0.0;
+    double tot = use_e ? te : tw;
+    if (tot <= 0.0) {
+        use_e = !use_e;
+        tot = use_e ? te : tw;
+    }
+    const double den = tot > 0.0 ? tot : 1.0;
+    const double* qs = use_e ? a.q_e : a.q_w;
+    for (int k = 0; k < a.n; ++k) out[k * pf + o] = out[k * pf + o] + R * __ldg(qs + k * pf + o) / den;
+}
+
+// The whole barotropic correction of 32 faces in one CTA (the first pass, up to `max_iter` Newton steps and the final
+// fluxes), for columns of up to LPT * W layers: lane = face, and each of the W warps keeps LPT layers of its faces, the
+// upwind side's edge value, slope and curvature in registers, the velocities and thickness limits in shared memory.  A
+// Newton step then reads nothing from memory: every warp evaluates its layers at the new correction, the fluxes go
+// through shared memory, and the first warp adds them and their derivatives over the layers in the reference's order
+// and takes the step of its lane's face.  A layer whose velocity changes sign reloads the other side.
+//
+// The reference stops when every face of the grid has converged, which a CTA cannot know: the launch with check = 0
+// runs max_iter steps and marks in `unconverged` each step after which one of its faces had not converged; the launch
+// with check = 1 finds the step the reference stops at and, where that is before max_iter, runs the CTA again up to
+// there.  A face whose correction comes out unchanged stays as it is (its state repeats), so a CTA whose faces are all
+// there leaves its loop.
+//
+// What bounds it: instruction issue in the layers' evaluation, and the sums over the layers, which only other CTAs'
+// work hides (CTAS of them fit an SM): 1.29 ms for 20 steps at 512 x 512 x 50.  As one launch per step, each re-reading
+// 0.63 GB, the 22 passes took 3.55 ms (158 us per step).
+template <int LPT, int W, int CTAS>
+__global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int max_iter, int check,
+                                                                  double* __restrict__ out)
+{
+    extern __shared__ double sh[];
+    constexpr int ROWS = LPT * W;                  // rows of 32 lanes: F, dF, u, limit (ROWS each), then
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, n = a.n;
+    double* shF = sh + lane;
+    double* shD = shF + 32 * ROWS;
+    double* shU = shD + 32 * ROWS;
+    double* shL = shU + 32 * ROWS;
+    double* row = shL + 32 * ROWS;                 // te, tw, du / R, den
+    __shared__ int command;                        // 1: evaluate at du; 0: done
+    int steps = max_iter;
+    if (check) {
+        int last = 0;                              // the reference's steps: up to the first that left no face
+        for (; last < max_iter; last += 32) {
+            const bool none = last + lane < max_iter && *(volatile int*)(a.unconverged + last + lane) == 0;
+            const unsigned first = __ballot_sync(0xffffffffu, none);
+            if (first) {
+                last += __ffs(first) - 1;
+                break;
+            }
+        }
+        if (last + 1 >= max_iter) return;
+        steps = last + 1;
+    }
+    const int nf = a.nx + 1, pf = a.ny * nf;
+    const int o = blockIdx.x * 32 + lane;
+    const bool in = o < pf;
+    const int oc = in ? o : pf - 1, j = oc / nf, f = oc - j * nf;
+    const FaceCells fc = face_cells(a, j, f);
+    const bool open = in && fc.aw && fc.ae;
+    const int k0 = wp * LPT;
+    // a closed face: width 1, velocity, edges and length 0, so that its fluxes come out +0
+    const double dxw = open ? fc.dxw : 1.0, dxe = open ? fc.dxe : 1.0, L_f = open ? __ldg(a.L + oc) : 0.0;
+    const double yw = shared_recip(dxw), ye = shared_recip(dxe);
+    double edge[LPT], dh[LPT], curv[LPT];
+    unsigned west = 0, limited = 0;                // bit l: layer k0 + l holds its west cell's values; has a limit
+
+    // the upwind cell's values of layer k0 + l
+    auto load_side = [&](int l, bool w) {
+        const int k = k0 + l, oo = k * a.T.pc + (w ? fc.cw : fc.ce);
+        const double hu = nan_to_num(__ldg(a.T.h + oo));
+        const double hw = __ldg(a.h_w + oo), he = __ldg(a.h_e + oo);
+        const double qq = __ldg((w ? a.q_e : a.q_w) + k * pf + oc);
+        edge[l] = w ? he : hw;
+        dh[l] = w ? hw - he : he - hw;
+        curv[l] = (hw + he) - 2.0 * hu;
+        west = w ? west | (1u << l) : west & ~(1u << l);
+        shL[k * 32] = qq < hu ? qq : INFINITY;     // pmin with +inf leaves the first argument
+        if (qq < hu) limited |= 1u << l;
+    };
+    // fluxes and their derivatives of this warp's layers at velocity u (+ du) into shared memory (face_flux)
+    auto evaluate = [&](double du, bool shift) {
+        unsigned turned = 0;                       // a velocity whose sign bit is not its side's (-0.0 among them)
+#pragma unroll
+        for (int l = 0; l < LPT; ++l)
+            if (k0 + l < n) {
+                const double v = shift ? shU[(k0 + l) * 32] + du : shU[(k0 + l) * 32];
+                turned |= (((unsigned)__double2hiint(v) >> 31) ^ (west >> l) ^ 1u) & 1u;
+            }
+        if (turned && open) {
+#pragma unroll
+            for (int l = 0; l < LPT; ++l)
+                if (k0 + l < n) {
+                    const bool w = (shift ? shU[(k0 + l) * 32] + du : shU[(k0 + l) * 32]) >= 0.0;
+                    if (w != (bool)((west >> l) & 1u)) load_side(l, w);
+                }
+        }
+        const unsigned some = __reduce_or_sync(0xffffffffu, limited);
+#pragma unroll
+        for (int l = 0; l < LPT; ++l) {
+            if (k0 + l >= n) break;
+            const int r = (k0 + l) * 32;
+            const double v = shift ? shU[r] + du : shU[r];
+            const bool w = v >= 0.0;
+            const double c = pmin(quot_rn(fabs(v) * a.dt, w ? dxw : dxe, w ? yw : ye), 1.0);
+            double mean = edge[l] + c * (0.5 * dh[l] + curv[l] * (c - 1.5));
+            double marg = edge[l] + c * (dh[l] + 3.0 * curv[l] * (c - 1.0));
+            if ((some >> l) & 1u) {
+                const double lim = shL[r];
+                mean = pmin(mean, lim);
+                marg = pmin(marg, lim);
+            }
+            shF[r] = L_f * v * pmax(mean, 0.0);
+            shD[r] = L_f * pmax(marg, 0.0);
+        }
+    };
+
+    // the velocities; the bracket over this warp's layers; whether the short quotients serve this CTA
+    const double limw = 0.5 * fc.dxw / a.dt, lime = 0.5 * fc.dxe / a.dt;
+    double mnw = INFINITY, mxe = -INFINITY;
+    auto mid = [](double x) {                      // |x| in [2^-250, 2^250): no quotient below leaves the range
+        return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (773u << 20) < (500u << 20);
+    };
+    bool odd = open && !(mid(dxw) && mid(dxe) && mid(a.dt) && yw != 0.0 && ye != 0.0 && a.dt > 0.0);
+#pragma unroll
+    for (int l = 0; l < LPT; ++l) {
+        edge[l] = dh[l] = curv[l] = 0.0;
+        if (k0 + l >= n) continue;
+        const double u = __ldg(a.ut + (k0 + l) * pf + oc);
+        mnw = pmin(mnw, limw - u);
+        mxe = pmax(mxe, -(lime + u));
+        odd = odd || (open && u != 0.0 && !mid(u));
+        shU[(k0 + l) * 32] = open ? u : 0.0;
+        shL[(k0 + l) * 32] = INFINITY;
+    }
+    if (__syncthreads_or(odd)) {
+        if (wp == 0 && in) ppm_face_general(a, o, steps, max_iter, !check, out);
+        return;
+    }
+    if (open) {
+#pragma unroll
+        for (int l = 0; l < LPT; ++l)
+            if (k0 + l < n) load_side(l, shU[(k0 + l) * 32] >= 0.0);
+    } else {
+        west = ~0u;
+    }
+    shF[wp * 32] = mnw;
+    shD[wp * 32] = mxe;
+    __syncthreads();
+    double hi, lo, du = 0.0, err = 0.0, ds = 0.0, s = 0.0, q = 0.0;       // the first warp's: its lanes' faces
+    if (wp == 0) {
+        mnw = INFINITY;
+        mxe = -INFINITY;
+        for (int w = 0; w < W; ++w) {
+            mnw = pmin(mnw, shF[w * 32]);
+            mxe = pmax(mxe, shD[w * 32]);
+        }
+        hi = pmax(pmin(limw, mnw), 0.0);
+        lo = pmin(pmax(-lime, mxe), 0.0);
+        q = in ? __ldg(a.Q_bt + oc) : 0.0;
+    } else if (wp >= W - 2) {                      // the face's transport thicknesses, for the residual's share
+        const double* qs = wp == W - 2 ? a.q_e : a.q_w;
+        double acc = 0.0;
+        for (int k = 0; k < n; ++k) acc += __ldg(qs + k * pf + oc);
+        row[(wp == W - 2 ? 0 : 1) * 32] = acc;
+    }
+    __syncthreads();
+    evaluate(0.0, steps == 0);
+    for (int it = -1;; ++it) {                     // it: the step just evaluated (-1: the given velocities)
+        __syncthreads();
+        if (wp == 0) {
+            double s2 = 0.0, d2 = 0.0;
+#pragma unroll 5
+            for (int k = 0; k < n; ++k) {
+                s2 += shF[k * 32];
+                d2 += shD[k * 32];
+            }
+            s = s2;
+            err = s2 - q;
+            ds = d2;
+            const bool left = in && fabs(err) > 1e-12 * pmax(fabs(q), 1.0);
+            if (it >= 0 && !check && __any_sync(0xffffffffu, left) && lane == 0) a.unconverged[it] = 1;
+            int go = 0;
+            if (it + 1 < steps) {
+                const double d = du;
+                if (err > 0.0) hi = d;
+                if (err < 0.0) lo = d;
+                const double step = ds > 0.0 ? -err / ds : 0.0;
+                double nw = d + step;
+                if (step > 0.0 && nw >= hi) nw = 0.5 * (d + hi);
+                if (step < 0.0 && nw <= lo) nw = 0.5 * (d + lo);
+                du = nw;
+                const bool moved = in && (it < 0 || __double_as_longlong(nw) != __double_as_longlong(d));
+                go = __any_sync(0xffffffffu, moved);
+                // every later step of these faces repeats the last one
+                if (!go && !check && __any_sync(0xffffffffu, left) && lane == 0)
+                    for (int m = it + 1; m < max_iter; ++m) a.unconverged[m] = 1;
+            }
+            if (go) {
+                row[2 * 32] = du;
+            } else {                               // the residual's share (cnuity.F90 style, ale.py:718-740)
+                const double R = q - s, te = row[0], tw = row[32];
+                bool use_e = R >= 0.0;
+                double tot = use_e ? te : tw;
+                if (tot <= 0.0) {
+                    use_e = !use_e;
+                    tot = use_e ? te : tw;
+                }
+                row[2 * 32] = R;
+                row[3 * 32] = tot > 0.0 ? tot : 1.0;
+                row[0] = use_e ? 1.0 : 0.0;
+            }
+            if (lane == 0) command = go;
+        }
+        __syncthreads();
+        if (!command) break;
+        evaluate(row[2 * 32], true);
+    }
+    // final fluxes
+    if (in) {
+        const double R = row[2 * 32], den = row[3 * 32], y = shared_recip(den);
+        const double* qs = row[0] != 0.0 ? a.q_e : a.q_w;
+#pragma unroll 1
+        for (int k = k0; k < k0 + LPT && k < n; ++k)
+            out[k * pf + o] = open ? shF[k * 32] + quotient(R * __ldg(qs + k * pf + o), den, y) : 0.0;
+    }
+}
+
+template <int LPT, int W, int CTAS>
+static cudaError_t ppm_newton_launch(const PPMArgs& a, int max_iter, double* out, cudaStream_t st)
+{
+    const unsigned g = (unsigned)(((i64)a.ny * (a.nx + 1) + 31) / 32);
+    constexpr size_t shmem = (size_t)(4 * LPT * W + 4) * 32 * sizeof(double);
+    const auto kernel = ppm_newton_kernel<LPT, W, CTAS>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
+    if (e != cudaSuccess) return e;
+    kernel<<<g, 32 * W, shmem, st>>>(a, max_iter, 0, out);
+    if (max_iter > 1) kernel<<<g, 32 * W, shmem, st>>>(a, max_iter, 1, out);
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -765,8 +1050,8 @@ extern "C" int pocean_ppm_edges_f64(const double* h, const uint8_t* active, int 
     rc = pocean_check_device();
     if (rc) return rc;
     const pr::Thick T{h, active, ny * nx, nx};
-    pr::ppm_edges_kernel<<<dim3((unsigned)((nx + 127) / 128), ny, nz), 128, 0, (cudaStream_t)stream>>>(T, nz, ny, h_min,
-                                                                                                      h_w, h_e);
+    const dim3 g((unsigned)ceil_div(nx, 30 * pr::EDGE_WARPS), ny, nz);
+    pr::ppm_edges_kernel<<<g, 32 * pr::EDGE_WARPS, 0, (cudaStream_t)stream>>>(T, nz, ny, h_min, h_w, h_e);
     return pocean_check_launch(fn);
 }
 
@@ -812,7 +1097,18 @@ extern "C" int pocean_ppm_transport_f64(const double* h, const double* ut, const
     a.dt = dt; a.n = nz; a.ny = ny; a.nx = nx;
     cudaError_t e = cudaMemsetAsync(a.unconverged, 0, (size_t)(max_iter + 1) * sizeof(int), st);
     if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
-    pr::ppm_edges_kernel<<<dim3((unsigned)((nx + 127) / 128), ny, nz), 128, 0, st>>>(a.T, nz, ny, 2e-10, h_w, h_e);
+    const dim3 ge((unsigned)ceil_div(nx, 30 * pr::EDGE_WARPS), ny, nz);
+    pr::ppm_edges_kernel<<<ge, 32 * pr::EDGE_WARPS, 0, st>>>(a.T, nz, ny, 2e-10, h_w, h_e);
+    if (nz <= 80) {
+        // layers per warp, warps, CTAs per SM: four warps and as many CTAs as registers and shared memory hold are the
+        // fastest split (whole layer-transport step at 512 x 512 x 50: 3.87 ms; 7 layers x 8 warps x 3 CTAs 4.44,
+        // 5 x 12 x 2 4.24, 10 x 5 x 3 3.98): what a CTA's sums leave idle, the other CTAs fill
+        e = nz <= 32 ? pr::ppm_newton_launch<8, 4, 5>(a, max_iter, Qx, st)
+                     : (nz <= 52 ? pr::ppm_newton_launch<13, 4, 4>(a, max_iter, Qx, st)
+                                 : pr::ppm_newton_launch<20, 4, 2>(a, max_iter, Qx, st));
+        if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
+        return pocean_check_launch(fn);
+    }
     const i64 nfaces = (i64)ny * (nx + 1);
     const unsigned g = (unsigned)((nfaces + 127) / 128);
     pr::ppm_init_kernel<<<g, 128, 0, st>>>(a);
