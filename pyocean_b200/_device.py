@@ -45,10 +45,13 @@ class Converter:
         return t.contiguous()
 
     def u8(self, a, shape: tuple) -> torch.Tensor:
-        """A boolean mask as a contiguous uint8 (0/1) tensor of ``shape`` on the device."""
+        """A boolean mask as a contiguous uint8 (0 / non-zero) tensor of ``shape`` on the device."""
         if isinstance(a, torch.Tensor):
             t = a.to(self.device, non_blocking=True)
-            t = t if t.dtype == torch.uint8 else (t != 0).to(torch.uint8)
+            if t.dtype == torch.bool:
+                t = t.view(torch.uint8)                    # one byte per cell, which the kernels test against 0
+            elif t.dtype != torch.uint8:
+                t = (t != 0).to(torch.uint8)
         else:
             t = torch.from_numpy(np.ascontiguousarray(np.asarray(a, dtype=bool)).view(np.uint8)).to(self.device)
         if tuple(t.shape) != tuple(shape):
