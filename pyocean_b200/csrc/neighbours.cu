@@ -13,6 +13,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "exactdiv.cuh"
 #include "remap_io.cuh"
 
 namespace po {
@@ -506,59 +507,55 @@ constexpr int DTI = 32, DTJ = 4, DKL = 4;
 #else
 #define DIFF_BOUNDS __launch_bounds__(DTI * DTJ)
 #endif
-__global__ void DIFF_BOUNDS diffuse_ale_kernel(const double* __restrict__ T,
-                                                                const double* __restrict__ Tw,
-                                                                const double* __restrict__ h,
-                                                                const uint8_t* __restrict__ act,
-                                                                const double* __restrict__ cx,
-                                                                const double* __restrict__ cy,
-                                                                const uint8_t* __restrict__ okx,
-                                                                const uint8_t* __restrict__ oky,
-                                                                const double* __restrict__ V, int nt, int n, int ny,
-                                                                int nx, bool per_x, bool per_y, double kh, double dt,
-                                                                double* __restrict__ out)
+// IX: 32-bit offsets within a layer from block-uniform layer bases (layers of fewer than 2^31 cells), or 64-bit ones.
+template <typename IX>
+__global__ void DIFF_BOUNDS diffuse_ale_kernel(const double* __restrict__ T, const double* __restrict__ Tw,
+                                               const double* __restrict__ h, const uint8_t* __restrict__ act,
+                                               const double* __restrict__ cx, const double* __restrict__ cy,
+                                               const uint8_t* __restrict__ okx, const uint8_t* __restrict__ oky,
+                                               const double* __restrict__ V, int nt, int n, int ny, int nx, bool per_x,
+                                               bool per_y, double kh, double dt, double* __restrict__ out)
 {
     const int i = blockIdx.x * DTI + threadIdx.x % DTI;
     const int j = blockIdx.y * DTJ + threadIdx.x / DTI;
     if (i >= nx || j >= ny) return;
     const int k0 = blockIdx.z * DKL, k1 = min(k0 + DKL, n);
     const i64 plane = (i64)ny * nx;
-    const i64 a = (i64)j * nx + i;
+    const IX a = (IX)j * nx + i;
     const bool has_w = (i > 0 || per_x), has_e = (i < nx - 1 || per_x);
     const bool has_s = (j > 0 || per_y), has_n = (j < ny - 1 || per_y);
     const int iw = i > 0 ? i - 1 : nx - 1, ie = i < nx - 1 ? i + 1 : 0;
     const int js = j > 0 ? j - 1 : ny - 1, jn = j < ny - 1 ? j + 1 : 0;
+    const IX aw = (IX)j * nx + iw, ae = (IX)j * nx + ie, as = (IX)js * nx + i, an = (IX)jn * nx + i;
     const i64 fw_i = (i64)j * (nx + 1) + i, fe_i = (i64)j * (nx + 1) + ie;
-    const i64 fs_i = (i64)j * nx + i, fn_i = (i64)jn * nx + i;
-    const i64 aw = (i64)j * nx + iw, ae = (i64)j * nx + ie, as = (i64)js * nx + i, an = (i64)jn * nx + i;
     const bool ow = has_w && __ldg(okx + fw_i), oe = has_e && __ldg(okx + fe_i);
-    const bool os = has_s && __ldg(oky + fs_i), on = has_n && __ldg(oky + fn_i);
+    const bool os = has_s && __ldg(oky + a), on = has_n && __ldg(oky + an);
     const bool ac = __ldg(act + a) != 0;
     const bool bw = __ldg(act + aw) && ac, be = ac && __ldg(act + ae);
     const bool bs = __ldg(act + as) && ac, bn = ac && __ldg(act + an);
-    const double cxw = __ldg(cx + fw_i), cxe = __ldg(cx + fe_i), cys = __ldg(cy + fs_i), cyn = __ldg(cy + fn_i);
-#pragma unroll 2
+    const double cxw = __ldg(cx + fw_i), cxe = __ldg(cx + fe_i), cys = __ldg(cy + a), cyn = __ldg(cy + an);
+#pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-        const i64 hk = (i64)k * plane;
-        const double hc = __ldg(h + hk + a), hw = __ldg(h + hk + aw), he = __ldg(h + hk + ae),
-                     hs = __ldg(h + hk + as), hn = __ldg(h + hk + an);
-        const double v = __ldg(V + hk + a);
-        const double hu_w = bw ? pmin(hw, hc) : 0.0;
-        const double hu_e = be ? pmin(hc, he) : 0.0;
-        const double hv_s = bs ? pmin(hs, hc) : 0.0;
-        const double hv_n = bn ? pmin(hc, hn) : 0.0;
+        const double* __restrict__ hk = h + k * plane;
+        const double hc = __ldg(hk + a), hw = __ldg(hk + aw), he = __ldg(hk + ae), hs = __ldg(hk + as),
+                     hn = __ldg(hk + an);
+        const double v = __ldg(V + k * plane + a);
+        // (-K_h L / dx) min(h_L, h_R), the same for every tracer
+        const double gw = -kh * cxw * (bw ? pmin(hw, hc) : 0.0), ge = -kh * cxe * (be ? pmin(hc, he) : 0.0);
+        const double gs = -kh * cys * (bs ? pmin(hs, hc) : 0.0), gn = -kh * cyn * (bn ? pmin(hc, hn) : 0.0);
+        const double y = shared_recip(v);
         for (int t = 0; t < nt; ++t) {
-            const i64 to = (i64)t * n * plane + hk;
-            const double* tw = Tw + to;
+            const i64 to = ((i64)t * n + k) * plane;
+            const double* __restrict__ tw = Tw + to;
             const double twc = __ldg(tw + a), tww = __ldg(tw + aw), twe = __ldg(tw + ae), tws = __ldg(tw + as),
                          twn = __ldg(tw + an);
             const double tc = __ldg(T + to + a);
-            const double fw = ow ? -kh * cxw * hu_w * (twc - tww) : 0.0;
-            const double fe = oe ? -kh * cxe * hu_e * (twe - twc) : 0.0;
-            const double fs = os ? -kh * cys * hv_s * (twc - tws) : 0.0;
-            const double fn = on ? -kh * cyn * hv_n * (twn - twc) : 0.0;
+            const double fw = ow ? gw * (twc - tww) : 0.0;
+            const double fe = oe ? ge * (twe - twc) : 0.0;
+            const double fs = os ? gs * (twc - tws) : 0.0;
+            const double fn = on ? gn * (twn - twc) : 0.0;
             const double div = fe - fw + fn - fs;
-            out[to + a] = v > 0.0 ? tc - dt * div / v : tc;
+            (out + to)[a] = v > 0.0 ? tc - quotient(dt * div, v, y) : tc;
         }
     }
 }
@@ -700,9 +697,10 @@ extern "C" int pocean_diffuse_ale_f64(const double* T, const double* Tw, const d
     if (rc) return rc;
     const dim3 grid((unsigned)((nx + nb::DTI - 1) / nb::DTI), (unsigned)((ny + nb::DTJ - 1) / nb::DTJ),
                     (unsigned)((nz + nb::DKL - 1) / nb::DKL));
-    nb::diffuse_ale_kernel<<<grid, nb::DTI * nb::DTJ, 0, (cudaStream_t)stream>>>(
-        T, Tw, h, act, cx, cy, okx, oky, V, nt, nz, ny, nx, (flags & POCEAN_PERIODIC_X) != 0,
-        (flags & POCEAN_PERIODIC_Y) != 0, kh, dt, out);
+    const auto kernel = (i64)ny * nx < (1ll << 31) ? nb::diffuse_ale_kernel<int> : nb::diffuse_ale_kernel<i64>;
+    kernel<<<grid, nb::DTI * nb::DTJ, 0, (cudaStream_t)stream>>>(T, Tw, h, act, cx, cy, okx, oky, V, nt, nz, ny, nx,
+                                                                 (flags & POCEAN_PERIODIC_X) != 0,
+                                                                 (flags & POCEAN_PERIODIC_Y) != 0, kh, dt, out);
     return pocean_check_launch(fn);
 }
 
