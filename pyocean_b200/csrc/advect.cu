@@ -40,40 +40,27 @@ constexpr int TI = 32;          // tile width (i, contiguous in memory)
 constexpr int TJ = 8;           // tile height (j)
 constexpr int NTHREADS = TI * TJ;
 
-// Launch bounds of the coefficient and final passes; POCEAN_*_CTAS (resident CTAs per SM) sets their register
-// budget when defined, else ptxas chooses.  The final pass is fitted to 4 CTAs (32 warps, 64 registers) per SM:
-// 1.5 % faster for the step than 3 CTAs, measured at 512 x 512 x 50; the coefficient pass keeps ptxas's choice
-// (5 CTAs, which spills, was slower).
+// Launch bounds of the coefficient and final passes; POCEAN_*_CTAS (resident CTAs per SM) sets their register budget.
+// Both are fitted to 4 CTAs (32 warps, 64 registers) per SM at 512 x 512 x 50: the step 3.55 ms, with the coefficient
+// pass at ptxas's choice (68 registers, 3 CTAs) 3.64, both at 5 / 6 CTAs 3.63 / 3.72.
+#ifndef POCEAN_COEFF_CTAS
+#define POCEAN_COEFF_CTAS 4
+#endif
 #ifndef POCEAN_FINAL_CTAS
 #define POCEAN_FINAL_CTAS 4
 #endif
-#ifdef POCEAN_COEFF_CTAS
 #define COEFF_BOUNDS __launch_bounds__(NTHREADS, POCEAN_COEFF_CTAS)
-#else
-#define COEFF_BOUNDS __launch_bounds__(NTHREADS)
-#endif
-#ifdef POCEAN_FINAL_CTAS
 #define FINAL_BOUNDS __launch_bounds__(NTHREADS, POCEAN_FINAL_CTAS)
-#else
-#define FINAL_BOUNDS __launch_bounds__(NTHREADS)
-#endif
-// The batched coefficient and final passes have budgets of their own (the domains of a batch usually carry one
-// tracer, so a thread's loop over the tracers runs once).  The batched coefficient pass at 6 CTAs per SM (40
-// registers, spilling to L1): the 64-domain batched step 40.92 ms against 42.99 ms at ptxas's choice (68 registers,
-// 3 CTAs), 41.14 / 41.16 ms at 4 / 5 CTAs; the batched final pass keeps the single-domain budget (5 CTAs: slower).
+// The batched passes have budgets of their own; fitted to 4 CTAs too (batch of 24 uneven domains, one tracer: 17.73 ms
+// against 17.90 with the coefficient pass at 6 CTAs, 18.49 with both at 5).
 #ifndef POCEAN_COEFF_BATCHED_CTAS
-#define POCEAN_COEFF_BATCHED_CTAS 6
+#define POCEAN_COEFF_BATCHED_CTAS 4
 #endif
-#ifdef POCEAN_COEFF_BATCHED_CTAS
+#ifndef POCEAN_FINAL_BATCHED_CTAS
+#define POCEAN_FINAL_BATCHED_CTAS 4
+#endif
 #define COEFF_BATCHED_BOUNDS __launch_bounds__(NTHREADS, POCEAN_COEFF_BATCHED_CTAS)
-#else
-#define COEFF_BATCHED_BOUNDS COEFF_BOUNDS
-#endif
-#ifdef POCEAN_FINAL_BATCHED_CTAS
 #define FINAL_BATCHED_BOUNDS __launch_bounds__(NTHREADS, POCEAN_FINAL_BATCHED_CTAS)
-#else
-#define FINAL_BATCHED_BOUNDS FINAL_BOUNDS
-#endif
 
 // ---------------------------------------------------------------------------------------------------------------
 // Donor-cell flux F_L of x-face gf (sigma_baroclinic.py:486-494; periodic: every face interior, face nx = face 0).
@@ -117,33 +104,39 @@ namespace po {
 
 
 // Pass 4: Zalesak R+ / R- (sigma_baroclinic.py:407-432): bounds over the cell, its x / y neighbours and the layers
-// k +- 1 (ok cells), P from the antidiffusive fluxes of the cell's faces, Q from V1 and c_L.
-__device__ __forceinline__ void coeff_body(const StepArgs& a, int i, int j, int k)
+// k +- 1 (ok cells), P from the antidiffusive fluxes of the cell's faces, Q from V1 and c_L.  INNER: the CTA's cells have
+// all their x / y neighbours inside the domain.
+template <bool INNER>
+__device__ __forceinline__ void coeff_cell(const StepArgs& a, int i, int j, int k)
 {
     const Shape s = a.s;
     const Flags fl(a.flags);
-    if (i >= s.nx || j >= s.ny) return;
     const double* cL = a.c1;
     // the 7-point stencil of the bounds: cell, x / y neighbours, layers k -+ 1 (ok cells only); its geometry is
-    // the same for every tracer
-    const int dk[7] = {0, 0, 0, 0, 0, -1, 1};
-    const int dj[7] = {0, 0, 0, -1, 1, 0, 0};
-    const int di[7] = {0, -1, 1, 0, 0, 0, 0};
-    // 32-bit offsets within a field (every field holds fewer than 2^31 entries)
+    // the same for every tracer.  32-bit offsets within a field (every field holds fewer than 2^31 entries).
     const int pl = s.ny * s.nx, gc = k * pl + j * s.nx + i;
     const bool self_ok = a.ok[gc];
-    int nb[7];
-#pragma unroll
-    for (int m = 0; m < 7; ++m) {
-        int kk = k + dk[m], jj = j + dj[m], ii = i + di[m];
-        bool in = kk >= 0 && kk < s.n;
-        if (fl.per_y) jj = wrap(jj, s.ny); else in = in && jj >= 0 && jj < s.ny;
-        if (fl.per_x) ii = wrap(ii, s.nx); else in = in && ii >= 0 && ii < s.nx;
-        const int o = in ? kk * pl + jj * s.nx + ii : 0;
-        nb[m] = (in && a.ok[o]) ? o : -1;
+    int nb[7] = {gc, gc - 1, gc + 1, gc - s.nx, gc + s.nx, k > 0 ? gc - pl : -1, k + 1 < s.n ? gc + pl : -1};
+    if (!INNER) {
+        if (i == 0) nb[1] = fl.per_x ? gc - 1 + s.nx : -1;
+        if (i == s.nx - 1) nb[2] = fl.per_x ? gc + 1 - s.nx : -1;
+        if (j == 0) nb[3] = fl.per_y ? gc - s.nx + pl : -1;
+        if (j == s.ny - 1) nb[4] = fl.per_y ? gc + s.nx - pl : -1;
     }
+#pragma unroll
+    for (int m = 0; m < 7; ++m)
+        if (nb[m] >= 0 && !a.ok[nb[m]]) nb[m] = -1;
     const double v1 = a.V1[gc];
     const int tstride = s.n * pl;
+    // the ok bytes say which values are read: their lines come meanwhile
+    for (int t = 0; t < s.nt; ++t) {
+        const i64 ci = plane_at(t, tstride) + gc;
+        const int p = t * s.n + k;
+        prefetch(a.C + ci);
+        prefetch(cL + ci);
+        prefetch(a.Sx + plane_at(p, s.ny * (s.nx + 1)) + (j * (s.nx + 1) + i));
+        prefetch(a.Sy + plane_at(p, (s.ny + 1) * s.nx) + (j * s.nx + i));
+    }
     for (int t = 0; t < s.nt; ++t) {
         const i64 ci = plane_at(t, tstride) + gc;
         double rin = 0.0, rout = 0.0;
@@ -170,12 +163,21 @@ __device__ __forceinline__ void coeff_body(const StepArgs& a, int i, int j, int 
             const double p_out = a.dt * (pmax(axe, 0.0) - pmin(axw, 0.0) + pmax(ayn, 0.0) - pmin(ays, 0.0));
             const double q_in = pmax(v1 * (cmax - cL[ci]), 0.0);
             const double q_out = pmax(v1 * (cL[ci] - cmin), 0.0);
-            rin = p_in > 0.0 ? pmin(1.0, q_in / p_in) : 0.0;
-            rout = p_out > 0.0 ? pmin(1.0, q_out / p_out) : 0.0;
+            // min(1, q / p): a quotient of q >= p is at least 1, so where the limiter does not bind no division runs
+            if (p_in > 0.0) rin = q_in >= p_in ? 1.0 : pmin(1.0, q_in / p_in);
+            if (p_out > 0.0) rout = q_out >= p_out ? 1.0 : pmin(1.0, q_out / p_out);
         }
         a.q1[ci] = rin;            // R+ (over the stencil classes)
         a.c2[ci] = rout;           // R- over c2
     }
+}
+
+// The cells of a 32 x 8 tile from (i0, j0).
+__device__ __forceinline__ void coeff_body(const StepArgs& a, int i0, int j0, int k)
+{
+    const int i = i0 + threadIdx.x % TI, j = j0 + threadIdx.x / TI;
+    if (i0 >= 1 && j0 >= 1 && i0 + TI < a.s.nx && j0 + TJ < a.s.ny) coeff_cell<true>(a, i, j, k);
+    else if (i < a.s.nx && j < a.s.ny) coeff_cell<false>(a, i, j, k);
 }
 
 // Face coefficient C of x-face f of row j (sigma_baroclinic.py:435-442): min(R+ downstream, R- upstream) by the
@@ -222,28 +224,42 @@ __device__ __forceinline__ double face_flux(bool interior, bool open, bool inflo
     return fl + 0.0 * A;
 }
 
-__device__ __forceinline__ void final_body(const StepArgs& a, int i, int j, int k)
+template <bool INNER>
+__device__ __forceinline__ void final_cell(const StepArgs& a, int i, int j, int k)
 {
     const Shape s = a.s;
     const Flags fl(a.flags);
-    if (i >= s.nx || j >= s.ny) return;
-    // neighbours (wrapped on periodic axes, -1 outside the domain) and which faces are interior
-    const int iw = fl.per_x ? wrap(i - 1, s.nx) : i - 1, ie = fl.per_x ? wrap(i + 1, s.nx) : (i + 1 < s.nx ? i + 1 : -1);
-    const int js = fl.per_y ? wrap(j - 1, s.ny) : j - 1, jn = fl.per_y ? wrap(j + 1, s.ny) : (j + 1 < s.ny ? j + 1 : -1);
-    const bool in_w = fl.per_x || i >= 1, in_e = fl.per_x || i + 1 <= s.nx - 1;
-    const bool in_s = fl.per_y || j >= 1, in_n = fl.per_y || j + 1 <= s.ny - 1;
+    const bool per_x = !INNER && fl.per_x, per_y = !INNER && fl.per_y;
+    // which faces are interior (INNER: the CTA's cells have all their neighbours inside the domain)
+    const bool in_w = INNER || per_x || i >= 1, in_e = INNER || per_x || i + 1 <= s.nx - 1;
+    const bool in_s = INNER || per_y || j >= 1, in_n = INNER || per_y || j + 1 <= s.ny - 1;
     // 32-bit offsets within a field (every field holds fewer than 2^31 entries)
     const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx;
     const int g = k * pl + j * s.nx + i, gx = k * xpl + j * (s.nx + 1) + i, gy = k * ypl + j * s.nx + i;
     const double v0 = __ldg(a.V0 + g), v1 = __ldg(a.V1 + g);
     const double qw = __ldg(a.Qx + gx);
-    const double qe = __ldg(a.Qx + ((fl.per_x && i + 1 == s.nx) ? gx + 1 - s.nx : gx + 1));
+    const double qe = __ldg(a.Qx + ((per_x && i + 1 == s.nx) ? gx + 1 - s.nx : gx + 1));
     const double qs = __ldg(a.Qy + gy);
-    const double qn = __ldg(a.Qy + ((fl.per_y && j + 1 == s.ny) ? gy - j * s.nx : gy + s.nx));
-    const i64 row = (i64)j * s.nx;
-    const i64 o_c = row + i, o_w = row + (iw >= 0 ? iw : i), o_e = row + (ie >= 0 ? ie : i);
-    const i64 o_s = (i64)(js >= 0 ? js : j) * s.nx + i, o_n = (i64)(jn >= 0 ? jn : j) * s.nx + i;
+    const double qn = __ldg(a.Qy + ((per_y && j + 1 == s.ny) ? gy - j * s.nx : gy + s.nx));
+    // the cell and its neighbours in a plane (wrapped on periodic axes, the cell itself outside the domain)
+    const int o_c = j * s.nx + i;
+    int o_w = o_c - 1, o_e = o_c + 1, o_s = o_c - s.nx, o_n = o_c + s.nx;
+    if (!INNER) {
+        if (i == 0) o_w = per_x ? o_w + s.nx : o_c;
+        if (i == s.nx - 1) o_e = per_x ? o_e - s.nx : o_c;
+        if (j == 0) o_s = per_y ? o_s + pl : o_c;
+        if (j == s.ny - 1) o_n = per_y ? o_n - pl : o_c;
+    }
     for (int t = 0; t < s.nt; ++t) {
+        if (t + 1 < s.nt) {                        // the next tracer's lines
+            const int p1 = (t + 1) * s.n + k;
+            const i64 c1 = plane_at(p1, pl) + o_c;
+            prefetch(a.C + c1);
+            prefetch(a.q1 + c1);
+            prefetch(a.c2 + c1);
+            prefetch(a.Sx + plane_at(p1, xpl) + (gx - k * xpl));
+            prefetch(a.Sy + plane_at(p1, ypl) + (gy - k * ypl));
+        }
         const int p = t * s.n + k;
         const i64 pc = plane_at(p, pl);
         const double* C = a.C + pc;
@@ -269,15 +285,23 @@ __device__ __forceinline__ void final_body(const StepArgs& a, int i, int j, int 
     }
 }
 
+// The cells of a 32 x 8 tile from (i0, j0).
+__device__ __forceinline__ void final_body(const StepArgs& a, int i0, int j0, int k)
+{
+    const int i = i0 + threadIdx.x % TI, j = j0 + threadIdx.x / TI;
+    if (i0 >= 1 && j0 >= 1 && i0 + TI < a.s.nx && j0 + TJ < a.s.ny) final_cell<true>(a, i, j, k);
+    else if (i < a.s.nx && j < a.s.ny) final_cell<false>(a, i, j, k);
+}
+
 // Single-domain launches of passes 4 and 5: a 32 x 8 tile of one layer per CTA.
 __global__ void COEFF_BOUNDS fct_coeff_kernel(StepArgs a)
 {
-    coeff_body(a, blockIdx.x * TI + threadIdx.x % TI, blockIdx.y * TJ + threadIdx.x / TI, a.k0 + blockIdx.z);
+    coeff_body(a, blockIdx.x * TI, blockIdx.y * TJ, a.k0 + blockIdx.z);
 }
 
 __global__ void FINAL_BOUNDS fct_final_kernel(StepArgs a)
 {
-    final_body(a, blockIdx.x * TI + threadIdx.x % TI, blockIdx.y * TJ + threadIdx.x / TI, a.k0 + blockIdx.z);
+    final_body(a, blockIdx.x * TI, blockIdx.y * TJ, a.k0 + blockIdx.z);
 }
 
 // Batched launches of passes 4 and 5: domain d owns CTAs off[d] .. off[d+1]-1, one 32 x 8 tile of one layer each.
@@ -287,7 +311,7 @@ __global__ void COEFF_BATCHED_BOUNDS fct_coeff_batched(const BatchDomain* __rest
     __shared__ BlockTile bt;
     __shared__ StepArgs sh;
     const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
-    coeff_body(a, bt.bx * TI + threadIdx.x % TI, bt.by * TJ + threadIdx.x / TI, bt.k);
+    coeff_body(a, bt.bx * TI, bt.by * TJ, bt.k);
 }
 
 __global__ void FINAL_BATCHED_BOUNDS fct_final_batched(const BatchDomain* __restrict__ doms,
@@ -296,7 +320,7 @@ __global__ void FINAL_BATCHED_BOUNDS fct_final_batched(const BatchDomain* __rest
     __shared__ BlockTile bt;
     __shared__ StepArgs sh;
     const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
-    final_body(a, bt.bx * TI + threadIdx.x % TI, bt.by * TJ + threadIdx.x / TI, bt.k);
+    final_body(a, bt.bx * TI, bt.by * TJ, bt.k);
 }
 
 // Effective flux F_L + C A of the step through u-face column face_i, (nt, n, ny) (tracers.py:251-254).
@@ -405,21 +429,6 @@ __device__ __forceinline__ double y_flux(const FacePlane& P, const Shape& s, con
     }
     if (f == 0) return fl.open_s ? q * (q > 0.0 ? P.e[o] : P.c[o]) : 0.0;
     return fl.open_n ? q * (q < 0.0 ? P.e[o - s.nx] : P.c[o - s.nx]) : 0.0;
-}
-
-// z-face flux through interface kf (between layers kf-1 and kf) of column (j, i): WENO5 in k on the layers of the
-// column, valid cells only, 0 on the bed and surface interfaces (sigma_baroclinic.py:335-353).
-template <bool ZV>
-__device__ __forceinline__ double z_flux(const StepArgs& a, const Shape& s, const double* cin, int t, int kf, int ij,
-                                         unsigned cls)
-{
-    if (a.Fz == nullptr || kf < 1 || kf > s.n - 1) return 0.0;
-    const int pl = s.ny * s.nx;                               // 32-bit offsets within a field
-    const double q = a.Fz[kf * pl + ij];
-    if (q == 0.0) return 0.0;
-    const bool pos = q >= 0.0;
-    return q * face_value<ZV, false, false>(cin + plane_at(t, s.n * pl), kf * pl + ij, pl, s.n, false, kf, pos,
-                                     (pos ? cls : cls >> 2) & 3u);
 }
 
 // Classes of the three faces of cell (k, j, i) (see face_class): bits 0-3 west, 4-7 south, 8-11 bottom.
@@ -552,13 +561,12 @@ __device__ __forceinline__ const double* rk3_stage_field(const StepArgs& a)
     return (STAGE <= 1 || STAGE == 4) ? a.C : ((STAGE == 2 || STAGE == 5) ? a.c1 : a.c2);
 }
 
-template <int STAGE, bool ZV, int FS>
-__device__ __forceinline__ void rk3_faces_body(const StepArgs& a, const uint16_t* __restrict__ classes, int t, int k,
-                                               int i, int j)
+// The upwind-3 / upwind-1 / centred faces of cell (t, k, j, i).
+template <int STAGE, int FS>
+__device__ __forceinline__ void rk3_lin_faces(const StepArgs& a, int t, int k, int i, int j)
 {
     const Shape s = a.s;
     const Flags fl(a.flags);
-    if (i >= s.nx || j >= s.ny) return;
     const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx, p = t * s.n + k;
     const i64 pc = plane_at(p, pl);
     const double* cin = rk3_stage_field<STAGE>(a);
@@ -571,29 +579,69 @@ __device__ __forceinline__ void rk3_faces_body(const StepArgs& a, const uint16_t
     double* sx = a.Sx + plane_at(p, xpl);
     double* sy = a.Sy + plane_at(p, ypl);
     const int fyo = j * s.nx + i, fxo = fyo + j;
-    if (FS != FS_WENO) {
-        sx[fxo] = x_face_lin<FS>(P, s, fl, j, i);
-        sy[fyo] = y_face_lin<FS>(P, s, fl, j, i);
-        a.Tx[pc + fyo] = zface_lin<FS>(a, s, cin, t, k, j, i);
-        if (i == s.nx - 1) sx[fxo + 1] = x_face_lin<FS>(P, s, fl, j, s.nx);
-        if (j == s.ny - 1) sy[fyo + s.nx] = y_face_lin<FS>(P, s, fl, s.ny, i);
-        return;
-    }
-    const unsigned cls = STAGE == 0 ? rk3_classes(a, s, fl, k, j, i) : __ldg(classes + plane_at(k, pl) + fyo);
-    const double fx = x_flux<ZV>(P, s, fl, j, i, cls);
-    sx[fxo] = fx;
-    if (fl.per_x && i == 0) sx[fxo + s.nx] = fx;                      // face nx of a periodic axis is face 0
-    const double fy = y_flux<ZV>(P, s, fl, j, i, cls >> 4);
-    sy[fyo] = fy;
-    if (fl.per_y && j == 0) sy[fyo + pl] = fy;
-    a.Tx[pc + fyo] = z_flux<ZV>(a, s, cin, t, k, fyo, cls >> 8);      // bottom interface k (0 at the bed)
-    if (i == s.nx - 1 && !fl.per_x) {
-        const double q = __ldg(P.qx + fxo + 1);
-        sx[fxo + 1] = fl.open_e ? q * (q < 0.0 ? P.e[fyo] : P.c[fyo]) : 0.0;
-    }
-    if (j == s.ny - 1 && !fl.per_y) {
-        const double q = __ldg(P.qy + fyo + s.nx);
-        sy[fyo + s.nx] = fl.open_n ? q * (q < 0.0 ? P.e[fyo] : P.c[fyo]) : 0.0;
+    sx[fxo] = x_face_lin<FS>(P, s, fl, j, i);
+    sy[fyo] = y_face_lin<FS>(P, s, fl, j, i);
+    a.Tx[pc + fyo] = zface_lin<FS>(a, s, cin, t, k, j, i);
+    if (i == s.nx - 1) sx[fxo + 1] = x_face_lin<FS>(P, s, fl, j, s.nx);
+    if (j == s.ny - 1) sy[fyo + s.nx] = y_face_lin<FS>(P, s, fl, s.ny, i);
+}
+
+// The WENO5 faces of cell (k, j, i) for tracers t0 .. t1-1; INNER: at least three cells from every horizontal edge (see
+// faces_cell).
+template <int STAGE, bool ZV, bool INNER>
+__device__ __forceinline__ void rk3_weno_faces(const StepArgs& a, const uint16_t* __restrict__ classes, int t0, int t1,
+                                               int k, int i, int j)
+{
+    const Shape s = a.s;
+    const Flags fl(a.flags);
+    const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx;
+    const int o = j * s.nx + i, ox = o + j;
+    const unsigned cls = STAGE == 0 ? rk3_classes(a, s, fl, k, j, i) : __ldg(classes + plane_at(k, pl) + o);
+    const double* __restrict__ qx = a.Qx + plane_at(k, xpl);
+    const double* __restrict__ qy = a.Qy + plane_at(k, ypl);
+    const double qw = __ldg(qx + ox), qs = __ldg(qy + o);
+    // bottom interface: between layers k - 1 and k of the column, 0 on the bed (sigma_baroclinic.py:335-353)
+    const double qb = a.Fz != nullptr && k >= 1 ? __ldg(a.Fz + plane_at(k, pl) + o) : 0.0;
+    const bool per_x = !INNER && fl.per_x, per_y = !INNER && fl.per_y;
+#pragma unroll 1
+    for (int t = t0; t < t1; ++t) {
+        const int p = t * s.n + k;
+        const i64 pc = plane_at(p, pl);
+        const double* __restrict__ c = rk3_stage_field<STAGE>(a) + pc;
+        double* sx = a.Sx + plane_at(p, xpl);
+        double* sy = a.Sy + plane_at(p, ypl);
+        double f = 0.0;
+        if (INNER || per_x || i >= 1) {
+            if (qw != 0.0) {
+                const bool pos = qw >= 0.0;
+                f = qw * face_value<ZV, false, INNER>(c, o, 1, s.nx, per_x, i, pos, (pos ? cls : cls >> 2) & 3u);
+            }
+        } else {
+            f = edge_flux<1>(fl.open_w, qw, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+        }
+        sx[ox] = f;
+        if (per_x && i == 0) sx[ox + s.nx] = f;                       // face nx of a periodic axis is face 0
+        f = 0.0;
+        if (INNER || per_y || j >= 1) {
+            if (qs != 0.0) {
+                const bool pos = qs >= 0.0;
+                f = qs * face_value<ZV, false, INNER>(c, o, s.nx, s.ny, per_y, j, pos, (pos ? cls >> 4 : cls >> 6) & 3u);
+            }
+        } else {
+            f = edge_flux<1>(fl.open_s, qs, c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+        }
+        sy[o] = f;
+        if (per_y && j == 0) sy[o + pl] = f;
+        f = 0.0;
+        if (qb != 0.0) {                                              // the column's layers are `pl` apart
+            const bool pos = qb >= 0.0;
+            f = qb * face_value<ZV, false, true>(c, o, pl, s.n, false, k, pos, (pos ? cls >> 8 : cls >> 10) & 3u);
+        }
+        (a.Tx + pc)[o] = f;
+        if (!INNER && i == s.nx - 1 && !per_x)
+            sx[ox + 1] = edge_flux<-1>(fl.open_e, __ldg(qx + ox + 1), c[o], a.inflow ? a.inflow[pc + o] : c[o]);
+        if (!INNER && j == s.ny - 1 && !per_y)
+            sy[o + s.nx] = edge_flux<-1>(fl.open_n, __ldg(qy + o + s.nx), c[o], a.inflow ? a.inflow[pc + o] : c[o]);
     }
 }
 
@@ -605,10 +653,17 @@ __device__ __forceinline__ void rk3_faces_body(const StepArgs& a, const uint16_t
 template <int STAGE, bool ZV, int FS, int TJR>
 __global__ void __launch_bounds__(TI * TJR, POCEAN_RK3_FACES_MINB * 256 / (TI * TJR)) rk3_faces_kernel(StepArgs a, const uint16_t* __restrict__ classes)
 {
-    int k, t;
-    split_plane(blockIdx.z, a.s.nt, a.tdiv, k, t);
-    rk3_faces_body<STAGE, ZV, FS>(a, classes, t, k, blockIdx.x * TI + threadIdx.x % TI,
-                                  blockIdx.y * TJR + threadIdx.x / TI);
+    const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJR, i = i0 + threadIdx.x % TI, j = j0 + threadIdx.x / TI;
+    int k, t0, t1;
+    split_tracers(a, k, t0, t1);
+    if (FS != FS_WENO) {
+        if (i < a.s.nx && j < a.s.ny)
+            for (int t = t0; t < t1; ++t) rk3_lin_faces<STAGE, FS>(a, t, k, i, j);
+    } else if (i0 >= 3 && j0 >= 3 && i0 + TI + 2 <= a.s.nx && j0 + TJR + 2 <= a.s.ny) {
+        rk3_weno_faces<STAGE, ZV, true>(a, classes, t0, t1, k, i, j);
+    } else if (i < a.s.nx && j < a.s.ny) {
+        rk3_weno_faces<STAGE, ZV, false>(a, classes, t0, t1, k, i, j);
+    }
 }
 
 template <int STAGE, int TJR>
@@ -982,19 +1037,20 @@ template <bool ZV, int FS>
 static void launch_rk3(const StepArgs& a, uint16_t* cls, bool pc, dim3 grid, cudaStream_t st)
 {
     constexpr int R = POCEAN_FACE_ROWS;
+    const dim3 fgrid(grid.x, grid.y, a.per_plane ? grid.z : a.s.n);
     if (FS == FS_WENO) rk3_class_kernel<R><<<dim3(grid.x, grid.y, a.s.n), TI * R, 0, st>>>(a, cls);
     if (pc) {
-        rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a, cls);
+        rk3_faces_kernel<4, false, FS_CEN, R><<<fgrid, TI * R, 0, st>>>(a, cls);
         rk3_update_kernel<4, R><<<grid, TI * R, 0, st>>>(a);
-        rk3_faces_kernel<5, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
+        rk3_faces_kernel<5, ZV, FS, R><<<fgrid, TI * R, 0, st>>>(a, cls);
         rk3_update_kernel<5, R><<<grid, TI * R, 0, st>>>(a);
         return;
     }
-    rk3_faces_kernel<1, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
+    rk3_faces_kernel<1, ZV, FS, R><<<fgrid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<1, R><<<grid, TI * R, 0, st>>>(a);
-    rk3_faces_kernel<2, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
+    rk3_faces_kernel<2, ZV, FS, R><<<fgrid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<2, R><<<grid, TI * R, 0, st>>>(a);
-    rk3_faces_kernel<3, ZV, FS, R><<<grid, TI * R, 0, st>>>(a, cls);
+    rk3_faces_kernel<3, ZV, FS, R><<<fgrid, TI * R, 0, st>>>(a, cls);
     rk3_update_kernel<3, R><<<grid, TI * R, 0, st>>>(a);
 }
 
@@ -1034,6 +1090,7 @@ extern "C" int pocean_advect_rk3_f64(const double* C, const double* V0, const do
     a.Sy = (double*)w;
     const dim3 grid(ceil_div(nx, TI), ceil_div(ny, POCEAN_FACE_ROWS), nt * nz);
     const bool pc = flags & POCEAN_TIME_PC;
+    a.per_plane = one_tracer_ctas(a.s, nz);
     if (flags & POCEAN_FACES_UP3) launch_rk3<false, FS_UP3>(a, cls, pc, grid, st);
     else if (flags & POCEAN_FACES_UP1) launch_rk3<false, FS_UP1>(a, cls, pc, grid, st);
     else if (flags & POCEAN_WENO_JS) launch_rk3<false, FS_WENO>(a, cls, pc, grid, st);
@@ -1122,7 +1179,8 @@ extern "C" int pocean_advect_rhs_f64(const double* c, const double* Qx, const do
     a.Sx = (double*)w; w += align_up((size_t)nt * nz * ny * (nx + 1) * sizeof(double));
     a.Sy = (double*)w;
     constexpr int R = POCEAN_FACE_ROWS;
-    const dim3 grid(ceil_div(nx, TI), ceil_div(ny, R), nt * nz);
+    a.per_plane = one_tracer_ctas(a.s, nz);
+    const dim3 grid(ceil_div(nx, TI), ceil_div(ny, R), a.per_plane ? nt * nz : nz);
     cudaStream_t st = (cudaStream_t)stream;
     if (centred) rk3_faces_kernel<4, false, FS_CEN, R><<<grid, TI * R, 0, st>>>(a, nullptr);
     else if (flags & POCEAN_FACES_UP3) rk3_faces_kernel<1, false, FS_UP3, R><<<grid, TI * R, 0, st>>>(a, nullptr);

@@ -52,4 +52,11 @@ __host__ __device__ __forceinline__ double pmin(double a, double b) { return (b 
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Starts bringing a line to L2 without a register for it: for loads that a thread can name early but issues late (after
+// a long chain, or behind the mask that says whether it needs them).  In the stage-3 face pass, the coefficient and the
+// final pass together 1.7 % of the step at 512 x 512 x 50 (3.56 -> 3.50 ms).
+#ifdef __CUDACC__
+__device__ __forceinline__ void prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+#endif
+
 }  // namespace po

@@ -193,6 +193,17 @@ __device__ __forceinline__ void faces_cell(const StepArgs& a, int t0, int t1, in
         double* sy = (STAGE == 2 ? a.Ty : a.Sy) + pv;
         const double* tx = a.Tx + pu;
         const double* ty = a.Ty + pv;
+        if (STAGE == 3) {                              // read after the WENO chains
+            prefetch(sx + ox);
+            prefetch(tx + ox);
+            prefetch(sy + o);
+            prefetch(ty + o);
+            prefetch(c0 + o);
+            if (t == t0) {
+                prefetch(a.V0 + plane_at(k, pl) + o);
+                prefetch(a.V1 + plane_at(k, pl) + o);
+            }
+        }
         double fw = 0.0, lw = 0.0, fs = 0.0, ls = 0.0;
         // west x-face
         if (INNER || per_x || i >= 1) {
@@ -283,13 +294,14 @@ __device__ __forceinline__ void faces_body(const StepArgs& a, int t0, int t1, in
 #ifndef POCEAN_FACES3_MINB
 #define POCEAN_FACES3_MINB 7
 #endif
-// The mixed-precision face passes (FP32 weights) hold fewer FP64 values: 7 blocks of 256 (1 % faster than 6; 5 and
-// 8 slower).
+// The mixed-precision face passes (FP32 weights) hold FP32 copies beside the FP64 values: 7 blocks of 256 for stages 1
+// and 2 and 6 (40 registers) for stage 3.  Four tracers of 512 x 512 x 75, the FCT step: 6.25 ms so, 6.52 with 7 for all,
+// 6.25 with 6 for all, 6.47 with 6 and 5.
 #ifndef POCEAN_FACES12_MINB_MIX
 #define POCEAN_FACES12_MINB_MIX 7
 #endif
 #ifndef POCEAN_FACES3_MINB_MIX
-#define POCEAN_FACES3_MINB_MIX 7
+#define POCEAN_FACES3_MINB_MIX 6
 #endif
 #define FACES12_BOUNDS(n) __launch_bounds__(n, (MIX ? POCEAN_FACES12_MINB_MIX : POCEAN_FACES12_MINB) * 256 / (n))
 #define FACES3_BOUNDS(n) __launch_bounds__(n, (MIX ? POCEAN_FACES3_MINB_MIX : POCEAN_FACES3_MINB) * 256 / (n))
