@@ -304,23 +304,17 @@ __global__ void FINAL_BOUNDS fct_final_kernel(StepArgs a)
     final_body(a, blockIdx.x * TI, blockIdx.y * TJ, a.k0 + blockIdx.z);
 }
 
-// Batched launches of passes 4 and 5: domain d owns CTAs off[d] .. off[d+1]-1, one 32 x 8 tile of one layer each.
-__global__ void COEFF_BATCHED_BOUNDS fct_coeff_batched(const BatchDomain* __restrict__ doms,
-                                                               const int* __restrict__ off, int ndom)
+// Batched launches of passes 4 and 5: one 32 x 8 tile of one layer of a domain per CTA.
+__global__ void COEFF_BATCHED_BOUNDS fct_coeff_batched(const __grid_constant__ FctBatch B)
 {
-    __shared__ BlockTile bt;
-    __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
-    coeff_body(a, bt.bx * TI, bt.by * TJ, bt.k);
+    const BlockTile bt = block_tile<false, TI, TJ>(B);
+    coeff_body(B.a[bt.d], bt.bx * TI, bt.by * TJ, bt.k);
 }
 
-__global__ void FINAL_BATCHED_BOUNDS fct_final_batched(const BatchDomain* __restrict__ doms,
-                                                               const int* __restrict__ off, int ndom)
+__global__ void FINAL_BATCHED_BOUNDS fct_final_batched(const __grid_constant__ FctBatch B)
 {
-    __shared__ BlockTile bt;
-    __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
-    final_body(a, bt.bx * TI, bt.by * TJ, bt.k);
+    const BlockTile bt = block_tile<false, TI, TJ>(B);
+    final_body(B.a[bt.d], bt.bx * TI, bt.by * TJ, bt.k);
 }
 
 // Effective flux F_L + C A of the step through u-face column face_i, (nt, n, ny) (tracers.py:251-254).
@@ -959,52 +953,65 @@ static int advect_fct_impl(const char* fn, bool mixed, const double* C, const do
 
 namespace po {
 
-// The FCT passes of every domain of a batch, one launch per pass (off_host: the CTA offsets also held on the device).
+// The CTA ranges of B's domains for a pass over TW x th tiles of their layers, or of their (t, k) planes; returns the
+// launch's CTAs.
+static unsigned batch_ranges(FctBatch& B, int th, bool planes)
+{
+    int total = 0;
+    for (int d = 0; d < B.ndom; ++d) {
+        const Shape& s = B.a[d].s;
+        const int tx = ceil_div(s.nx, TI), ty = ceil_div(s.ny, th), count = planes ? s.n * s.nt : s.n;
+        B.off[d] = total;
+        B.per_layer[d] = tile_magic((long long)tx * ty, count);
+        B.per_row[d] = tile_magic(tx, ty);
+        total += tx * ty * count;
+    }
+    B.off[B.ndom] = total;
+    return (unsigned)total;
+}
+
 template <bool ZV, bool MIX, int TJR>
-static void fct_batched_stages(const BatchDomain* doms, const int* po, unsigned np, const int* lo, unsigned nl, int ndom,
+static void fct_batched_stages(FctBatch& B, cudaStream_t st)
+{
+    const unsigned layers = batch_ranges(B, TJR, false);
+    fct_faces_batched<1, ZV, MIX, TJR><<<layers, TI * TJR, 0, st>>>(B);
+    unsigned planes = batch_ranges(B, TJR, true);
+    fct_update_batched<1, TJR><<<planes, TI * TJR, 0, st>>>(B);
+    batch_ranges(B, TJR, false);
+    fct_faces_batched<2, ZV, MIX, TJR><<<layers, TI * TJR, 0, st>>>(B);
+    planes = batch_ranges(B, TJR, true);
+    fct_update_batched<2, TJR><<<planes, TI * TJR, 0, st>>>(B);
+    batch_ranges(B, TJR, false);
+    fct_faces3_batched<ZV, MIX, TJR><<<layers, TI * TJR, 0, st>>>(B);
+}
+
+template <bool ZV, bool MIX>
+static void fct_batched_impl(FctBatch& B, int tile_rows, cudaStream_t st)
+{
+    const unsigned classes = batch_ranges(B, CLASS_ROWS, false);
+    fct_class_batched<<<classes, TI / 4 * CLASS_ROWS, 0, st>>>(B);
+    if (tile_rows == 4) fct_batched_stages<ZV, MIX, 4>(B, st);
+    else if (tile_rows == 16) fct_batched_stages<ZV, MIX, 16>(B, st);
+    else fct_batched_stages<ZV, MIX, 8>(B, st);
+    const unsigned tiles = batch_ranges(B, TJ, false);
+    fct_coeff_batched<<<tiles, NTHREADS, 0, st>>>(B);
+    fct_final_batched<<<tiles, NTHREADS, 0, st>>>(B);
+}
+
+// The FCT passes of every domain of a batch, one launch per pass and BATCH_CAP domains.
+cudaError_t fct_batched_launch(const BatchDomain* doms_host, int ndom, bool zv, bool mixed, int tile_rows,
                                cudaStream_t st)
 {
-    fct_faces_batched<1, ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
-    fct_update_batched<1, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
-    fct_faces_batched<2, ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
-    fct_update_batched<2, TJR><<<np, TI * TJR, 0, st>>>(doms, po, ndom);
-    fct_faces3_batched<ZV, MIX, TJR><<<nl, TI * TJR, 0, st>>>(doms, lo, ndom);
-}
-
-// The FCT passes of every domain of a batch, one launch per pass (off_host: the CTA offsets also held on the device).
-template <bool ZV, bool MIX>
-static void fct_batched_impl(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int tile_rows,
-                             cudaStream_t st)
-{
-    const int* po = off_dev + BP_PTILE * (ndom + 1);
-    const int* lo = off_dev + BP_LTILE * (ndom + 1);
-    const int* to = off_dev + BP_TILE * (ndom + 1);
-    const unsigned np = (unsigned)off_host[BP_PTILE * (ndom + 1) + ndom];
-    const unsigned nl = (unsigned)off_host[BP_LTILE * (ndom + 1) + ndom];
-    const unsigned nt = (unsigned)off_host[BP_TILE * (ndom + 1) + ndom];
-    fct_class_batched<<<nt, NTHREADS / 4, 0, st>>>(doms, to, ndom);
-    if (tile_rows == 4) fct_batched_stages<ZV, MIX, 4>(doms, po, np, lo, nl, ndom, st);
-    else if (tile_rows == 16) fct_batched_stages<ZV, MIX, 16>(doms, po, np, lo, nl, ndom, st);
-    else fct_batched_stages<ZV, MIX, 8>(doms, po, np, lo, nl, ndom, st);
-    fct_coeff_batched<<<nt, NTHREADS, 0, st>>>(doms, to, ndom);
-    fct_final_batched<<<nt, NTHREADS, 0, st>>>(doms, to, ndom);
-}
-
-void fct_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, bool zv,
-                        bool mixed, int tile_rows, cudaStream_t st)
-{
-    if (zv && !mixed) fct_batched_impl<true, false>(doms, off_dev, off_host, ndom, tile_rows, st);
-    else if (!zv && !mixed) fct_batched_impl<false, false>(doms, off_dev, off_host, ndom, tile_rows, st);
-    else if (zv) fct_batched_impl<true, true>(doms, off_dev, off_host, ndom, tile_rows, st);
-    else fct_batched_impl<false, true>(doms, off_dev, off_host, ndom, tile_rows, st);
-}
-
-// CTAs of each batched FCT pass for one domain (see BatchPass).
-void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& layer_ctas, int& tile_ctas)
-{
-    layer_ctas = ceil_div(s.nx, TI) * ceil_div(s.ny, tile_rows) * s.n;
-    plane_ctas = layer_ctas * s.nt;
-    tile_ctas = ceil_div(s.nx, TI) * ceil_div(s.ny, TJ) * s.n;
+    FctBatch B;
+    for (int d0 = 0; d0 < ndom; d0 += BATCH_CAP) {
+        B.ndom = ndom - d0 < BATCH_CAP ? ndom - d0 : BATCH_CAP;
+        for (int d = 0; d < B.ndom; ++d) B.a[d] = doms_host[d0 + d].a;
+        if (zv && !mixed) fct_batched_impl<true, false>(B, tile_rows, st);
+        else if (!zv && !mixed) fct_batched_impl<false, false>(B, tile_rows, st);
+        else if (zv) fct_batched_impl<true, true>(B, tile_rows, st);
+        else fct_batched_impl<false, true>(B, tile_rows, st);
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace po

@@ -1,8 +1,9 @@
 // Batched ALE tracer steps of many independent domains: every pass of the FCT advection and the remap is one launch
 // over all domains (domain d owns a contiguous range of the launch's CTAs, found by binary search of a CTA-offset
-// table), so a batch of uneven domains costs 10-11 launches per step instead of 10-11 per domain, and the step
-// sequence can be captured in one CUDA graph.  The batch plan (descriptors of both ping-pong parities and the
-// offset tables) lives in a caller-provided device buffer; the library allocates no device memory.
+// table), so a batch of uneven domains costs 8-11 launches per step instead of as many per domain, and the step
+// sequence can be captured in one CUDA graph.  The FCT passes take their domains' arguments as kernel parameters, 64
+// domains a launch (FctBatch); the remap's descriptors of both ping-pong parities and its offset tables lie in a
+// caller-provided device buffer.  The library allocates no device memory.
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -21,6 +22,7 @@ struct pocean_batch {
     BatchDomain* dev_doms;             // 2 * ndom descriptors: parity 0 then parity 1
     int* dev_off;                      // BP_COUNT * (ndom + 1) offsets
     std::vector<int> host_off;
+    std::vector<BatchDomain> host_doms;    // 2 * ndom
 };
 
 extern "C" size_t pocean_batch_device_bytes(int ndom)
@@ -48,12 +50,14 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     std::vector<int> off((size_t)BP_COUNT * (ndom + 1), 0);
     const bool zv = !(domains[0].flags & POCEAN_WENO_JS);
     int nmax = 1;
-    for (int d = 0; d < ndom; ++d) nmax = domains[d].nz > nmax ? domains[d].nz : nmax;
     long long all_columns = 0;
-    for (int d = 0; d < ndom; ++d) all_columns += (long long)domains[d].ny * domains[d].nx * domains[d].nt;
+    for (int d = 0; d < ndom; ++d) {
+        nmax = domains[d].nz > nmax ? domains[d].nz : nmax;
+        all_columns += (long long)domains[d].ny * domains[d].nx * domains[d].nt;
+    }
     const bool segments = remap_batch_segments(all_columns, nmax);
     const int columns = remap_batched_columns(segments);
-    long long tot[BP_COUNT] = {};
+    long long tot[BP_COUNT] = {}, tiles = 0;
     for (int d = 0; d < ndom; ++d) {
         const pocean_domain& D = domains[d];
         if (D.nt < 1 || D.nz < 1 || D.ny < 1 || D.nx < 1 || (long long)D.nt * D.nz > 65535 || D.nz > 256)
@@ -72,6 +76,8 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
         const size_t need = pocean_advect_fct_workspace_bytes(D.nt, D.nz, D.ny, D.nx);
         if (!D.workspace || D.workspace_bytes < need || ((uintptr_t)D.workspace & 255))
             return pocean_fail(POCEAN_EWORKSPACE, "%s: domain %d: workspace of %zu bytes needed", fn, d, need);
+        tiles += ((long long)D.nx + 31) / 32 * (((long long)D.ny + tile_rows - 1) / tile_rows) * D.nt * D.nz;
+        if (tiles >= (1ll << 31)) return pocean_fail(POCEAN_EINVAL, "%s: batch too large for one launch", fn);
         for (int parity = 0; parity < 2; ++parity) {
             BatchDomain& B = host[(size_t)parity * ndom + d];
             std::memset(&B, 0, sizeof(B));
@@ -86,11 +92,9 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
             B.a.out = D.C_adv;
             B.h_src = D.h_src; B.h_tgt = D.h_tgt; B.wet = D.wet; B.remap_scheme = D.remap_scheme;
             B.rout = parity == 0 ? D.C_next : const_cast<double*>(D.C);
-            int pc, lc, tc;
-            fct_batched_ctas(B.a.s, tile_rows, pc, lc, tc);
             if (parity == 0) {
                 const long long cb = ((long long)D.ny * D.nx + columns - 1) / columns;
-                const long long n_pass[BP_COUNT] = {pc, lc, tc, cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt};
+                const long long n_pass[BP_COUNT] = {cb * (D.nt / 2), cb * (D.nt % 2), cb * D.nt};
                 for (int q = 0; q < BP_COUNT; ++q) {
                     off[(size_t)q * (ndom + 1) + d] = (int)tot[q];
                     tot[q] += n_pass[q];
@@ -110,6 +114,7 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     b->dev_doms = (BatchDomain*)device_buf;
     b->dev_off = (int*)((char*)device_buf + (((size_t)2 * ndom * sizeof(BatchDomain) + 255) & ~(size_t)255));
     b->host_off = off;
+    b->host_doms = host;
     // Pageable sources: each copy is staged before the call returns, so the host vectors may go; on the device
     // the copies are ordered after the work already on `stream` (which may still read an older plan here).
     cudaStream_t st = (cudaStream_t)stream;
@@ -133,9 +138,10 @@ extern "C" int pocean_batch_step(const pocean_batch* b, int parity, int remap_nf
     if (remap_nf != 1 && remap_nf != 2) return pocean_fail(POCEAN_EINVAL, "%s: remap_nf must be 1 or 2", fn);
     cudaStream_t st = (cudaStream_t)stream;
     const BatchDomain* doms = b->dev_doms + (size_t)parity * b->ndom;
-    fct_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, b->zv, mixed != 0, b->tile_rows, st);
-    const cudaError_t e = remap_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, remap_nf, b->nmax,
-                                               b->segments, st);
+    cudaError_t e = fct_batched_launch(b->host_doms.data() + (size_t)parity * b->ndom, b->ndom, b->zv, mixed != 0,
+                                       b->tile_rows, st);
+    if (e == cudaSuccess)
+        e = remap_batched_launch(doms, b->dev_off, b->host_off.data(), b->ndom, remap_nf, b->nmax, b->segments, st);
     if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
     return pocean_check_launch(fn);
 }

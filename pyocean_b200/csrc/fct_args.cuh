@@ -43,13 +43,11 @@ struct StepArgs {
     int k0;                             // first layer of a layer-range launch of the single-domain passes (else 0)
     unsigned tdiv;                      // plane_magic(s.nt): plane index -> layer without an integer division
     int per_plane;                      // single-domain face CTAs take one (tracer, layer) plane each (split_tracers)
-    int pad_;                           // (copied in 8-byte words)
     double* fx_face;
 };
 
 // One domain of a batch: its FCT arguments (a.C the stack, a.out the advected stack, a.q1.. its workspace) and
-// the remap of the advected stack onto its target grid (into rout).  nstrips / nsegs: its strip decomposition for
-// the batch's segment length.
+// the remap of the advected stack onto its target grid (into rout).
 struct BatchDomain {
     StepArgs a;
     const double* h_src;
@@ -67,14 +65,9 @@ __device__ __forceinline__ void split_plane(int p, int nt, unsigned tdiv, int& k
     t = p - k * nt;
 }
 
-// CTA offsets of every batched pass: domain d owns CTAs off[d] .. off[d+1]-1 of the launch (ndom + 1 entries each).
-enum BatchPass {
-    BP_PTILE = 0,       // tile_rows tiles of the (tracer, layer) planes: cell passes
-    BP_LTILE,           // tile_rows tiles of the layers: face passes
-    BP_TILE,            // 8-row tiles of the layers: class, coefficient and final passes
-    BP_RPAIR, BP_RREM, BP_RALL,     // column groups x field pairs, odd fields, all fields: remap
-    BP_COUNT
-};
+// CTA offsets of the batched remap launches: domain d owns CTAs off[d] .. off[d+1]-1 of the launch (ndom + 1 entries
+// each), for column groups x field pairs, odd fields, all fields.
+enum BatchPass { BP_RPAIR = 0, BP_RREM, BP_RALL, BP_COUNT };
 
 // The domain whose CTA range holds CTA b (binary search of off[0..ndom]).
 __device__ __forceinline__ int find_domain(const int* __restrict__ off, int ndom, int b)
@@ -88,27 +81,43 @@ __device__ __forceinline__ int find_domain(const int* __restrict__ off, int ndom
     return lo;
 }
 
-// The argument block of the block's domain, copied once into shared memory (every thread of a batched CTA works on
-// the same domain; reading the block from there is cheaper than a per-thread copy of ~200 bytes).  Call before any
-// thread returns: it contains a block barrier.
-__device__ __forceinline__ const StepArgs& block_args(const BatchDomain* __restrict__ doms, int d, StepArgs& sh)
+// A batched FCT launch: its domains' argument blocks and CTA ranges, passed as the kernel's parameter.  Parameters lie in
+// constant memory, so a CTA's search for its domain, its tile and every argument it reads are the same for all its
+// threads to the compiler and stay in uniform registers, as in a single-domain launch.  (Read from a device table
+// through shared memory they cost a batched step 11 % more than the single-domain calls, and each CTA the latency of the
+// search.)  Batches of more domains take several launches.
+constexpr int BATCH_CAP = 64;
+struct FctBatch {
+    int ndom;
+    int off[BATCH_CAP + 1];                       // domain d owns CTAs off[d] .. off[d+1]-1
+    unsigned long long per_layer[BATCH_CAP];      // tile_magic of the tiles of a layer and of a row of tiles
+    unsigned long long per_row[BATCH_CAP];
+    StepArgs a[BATCH_CAP];
+};
+static_assert(sizeof(FctBatch) <= 32000, "kernel parameters hold 32764 bytes");
+
+// x / d for 0 <= x < d count as a multiply: with m = ceil(2^47 / d), e = m d - 2^47 < d, floor(x m / 2^47) = x / d
+// whenever x e < 2^47 (Granlund & Montgomery 1994), which d d count < 2^47 ensures, and x m < 2^47 count fits 64 bits
+// (count <= 65535).  Else 0: the division itself.
+inline unsigned long long tile_magic(long long d, long long count)
 {
-    static_assert(sizeof(StepArgs) % sizeof(unsigned long long) == 0, "StepArgs is copied in 8-byte words");
-    constexpr int W = sizeof(StepArgs) / sizeof(unsigned long long);
-    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&doms[d].a);
-    unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sh);
-    for (int w = threadIdx.x; w < W; w += blockDim.x) dst[w] = __ldg(src + w);
-    __syncthreads();
-    return sh;
+    constexpr unsigned long long one = 1ull << 47;
+    if ((double)d * (double)d * (double)count >= 1.4e14) return 0ull;
+    return (one + (unsigned long long)d - 1) / (unsigned long long)d;
+}
+
+__device__ __forceinline__ int tile_div(int x, unsigned long long m, int d)
+{
+    return m ? (int)(((unsigned long long)(unsigned)x * m) >> 47) : x / d;
 }
 
 // The FCT workspace cut into a's buffers (advect.cu).
 void carve_fct_workspace(StepArgs& a, void* workspace);
 
-// Host launchers of the batched passes (advect.cu, remap.cu).
-void fct_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, bool zv,
-                        bool mixed, int tile_rows, cudaStream_t st);
-void fct_batched_ctas(const Shape& s, int tile_rows, int& plane_ctas, int& layer_ctas, int& tile_ctas);
+// Host launchers of the batched passes (advect.cu, remap.cu).  doms: the step's argument blocks, on the host and (for
+// the remap) on the device.
+cudaError_t fct_batched_launch(const BatchDomain* doms_host, int ndom, bool zv, bool mixed, int tile_rows,
+                               cudaStream_t st);
 bool remap_batch_segments(long long columns, int nmax);
 int remap_batched_columns(bool segments);
 cudaError_t remap_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int nf_mode,

@@ -345,72 +345,56 @@ __global__ void __launch_bounds__(TI * TJR) fct_class_kernel(StepArgs a)
     class_body(a, a.k0 + blockIdx.z, 4 * (blockIdx.x * TI + threadIdx.x % TI), blockIdx.y * TJR + threadIdx.x / TI);
 }
 
-// Where a batched CTA works (domain d owns CTAs off[d] .. off[d+1]-1): its domain d, its layer k (and
-// tracer t) and its 32 x TJR tile (bx, by).  The first thread of the CTA works it out (a binary search over the domains' CTA offsets and two integer
-// divisions, the same for every thread of the CTA) and shares it, with the domain's argument block, through shared
-// memory: done by every thread, that set-up cost the batched cell passes as many instructions again as their own work.
+// Where a batched CTA works: its domain's arguments, its layer k (and tracer t) and its TW x TH tile (bx, by).  PLANES:
+// the domain's CTAs count tiles of the (t, k) planes (k-major: the cell passes); else tiles of the layers (t = 0).
 struct BlockTile {
     int d, t, k, bx, by;
 };
 
-// The CTA's tile (bt) and its domain's argument block (sh), both in shared memory.  PLANES: the CTA's index counts
-// tiles of the (t, k) planes (k-major: the cell passes); else tiles of the layers (t = 0).  Call before any thread
-// returns: it contains block barriers.
-template <bool PLANES, int TJR>
-__device__ __forceinline__ const StepArgs& block_tile(const BatchDomain* __restrict__ doms, const int* __restrict__ off,
-                                                      int ndom, BlockTile& bt, StepArgs& sh)
+template <bool PLANES, int TW, int TH>
+__device__ __forceinline__ BlockTile block_tile(const FctBatch& B)
 {
-    if (threadIdx.x == 0) {
-        const int d = find_domain(off, ndom, blockIdx.x);
-        const Shape s = doms[d].a.s;
-        const int tx = ceil_div(s.nx, TI), ty = ceil_div(s.ny, TJR);
-        int local = blockIdx.x - __ldg(off + d);
-        const int p = local / (tx * ty);
-        local -= p * tx * ty;
-        int t = 0, k = p;
-        if (PLANES) split_plane(p, s.nt, doms[d].a.tdiv, k, t);
-        const int by = local / tx;
-        bt.d = d;
-        bt.t = t;
-        bt.k = k;
-        bt.by = by;
-        bt.bx = local - by * tx;
+    int lo = 0, hi = B.ndom - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (B.off[mid] <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
     }
-    __syncthreads();
-    return block_args(doms, bt.d, sh);
+    BlockTile bt;
+    bt.d = lo;
+    const Shape s = B.a[lo].s;
+    const int tx = ceil_div(s.nx, TW), tiles = tx * ceil_div(s.ny, TH), local = blockIdx.x - B.off[lo];
+    const int p = tile_div(local, B.per_layer[lo], tiles), rest = local - p * tiles;
+    bt.t = 0;
+    bt.k = p;
+    if (PLANES) split_plane(p, s.nt, B.a[lo].tdiv, bt.k, bt.t);
+    bt.by = tile_div(rest, B.per_row[lo], tx);
+    bt.bx = rest - bt.by * tx;
+    return bt;
 }
 
 template <int STAGE, bool ZV, bool MIX, int TJR>
-__device__ __forceinline__ void faces_batched_body(const BatchDomain* __restrict__ doms, const int* __restrict__ off,
-                                                   int ndom)
+__global__ void FACES12_BOUNDS(TI * TJR) fct_faces_batched(const __grid_constant__ FctBatch B)
 {
-    __shared__ BlockTile bt;
-    __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<false, TJR>(doms, off, ndom, bt, sh);
+    const BlockTile bt = block_tile<false, TI, TJR>(B);
+    const StepArgs& a = B.a[bt.d];
     faces_body<STAGE, ZV, MIX, TJR>(a, 0, a.s.nt, bt.k, bt.bx * TI, bt.by * TJR);
 }
 
-template <int STAGE, bool ZV, bool MIX, int TJR>
-__global__ void FACES12_BOUNDS(TI * TJR) fct_faces_batched(const BatchDomain* __restrict__ doms,
-                                                           const int* __restrict__ off, int ndom)
-{
-    faces_batched_body<STAGE, ZV, MIX, TJR>(doms, off, ndom);
-}
-
 template <bool ZV, bool MIX, int TJR>
-__global__ void FACES3_BOUNDS(TI * TJR) fct_faces3_batched(const BatchDomain* __restrict__ doms,
-                                                           const int* __restrict__ off, int ndom)
+__global__ void FACES3_BOUNDS(TI * TJR) fct_faces3_batched(const __grid_constant__ FctBatch B)
 {
-    faces_batched_body<3, ZV, MIX, TJR>(doms, off, ndom);
+    const BlockTile bt = block_tile<false, TI, TJR>(B);
+    const StepArgs& a = B.a[bt.d];
+    faces_body<3, ZV, MIX, TJR>(a, 0, a.s.nt, bt.k, bt.bx * TI, bt.by * TJR);
 }
 
-__global__ void __launch_bounds__(NTHREADS / 4) fct_class_batched(const BatchDomain* __restrict__ doms,
-                                                              const int* __restrict__ off, int ndom)
+// Tiles of the batched class pass: 32 x 32 cells by 256 threads of four cells each.
+constexpr int CLASS_ROWS = 32;
+__global__ void __launch_bounds__(TI / 4 * CLASS_ROWS) fct_class_batched(const __grid_constant__ FctBatch B)
 {
-    __shared__ BlockTile bt;
-    __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<false, TJ>(doms, off, ndom, bt, sh);
-    class_body(a, bt.k, bt.bx * TI + 4 * (threadIdx.x % (TI / 4)), bt.by * TJ + threadIdx.x / (TI / 4));
+    const BlockTile bt = block_tile<false, TI, CLASS_ROWS>(B);
+    class_body(B.a[bt.d], bt.k, bt.bx * TI + 4 * (threadIdx.x % (TI / 4)), bt.by * CLASS_ROWS + threadIdx.x / (TI / 4));
 }
 
 // Cell pass of stage STAGE = 1, 2 (sigma_baroclinic.py:452-468 `_fct_stage`); stage 3 has none (its face pass
@@ -455,13 +439,10 @@ __global__ void __launch_bounds__(TI * TJR) fct_update_kernel(StepArgs a)
 }
 
 template <int STAGE, int TJR>
-__global__ void __launch_bounds__(TI * TJR) fct_update_batched(const BatchDomain* __restrict__ doms,
-                                                               const int* __restrict__ off, int ndom)
+__global__ void __launch_bounds__(TI * TJR) fct_update_batched(const __grid_constant__ FctBatch B)
 {
-    __shared__ BlockTile bt;
-    __shared__ StepArgs sh;
-    const StepArgs& a = block_tile<true, TJR>(doms, off, ndom, bt, sh);
-    update_body<STAGE>(a, bt.t, bt.k, bt.bx * TI + threadIdx.x % TI, bt.by * TJR + threadIdx.x / TI);
+    const BlockTile bt = block_tile<true, TI, TJR>(B);
+    update_body<STAGE>(B.a[bt.d], bt.t, bt.k, bt.bx * TI + threadIdx.x % TI, bt.by * TJR + threadIdx.x / TI);
 }
 
 }  // namespace po
