@@ -21,6 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from .step import FCT_LAUNCHES, remap_launches
 
 
 class _Domain(ctypes.Structure):
@@ -146,12 +147,8 @@ class DomainBatch:
 
     @property
     def launches_per_step(self) -> int:
-        """The stencil classes, 3 face and 2 cell passes, the limiter coefficients, the final update, then the remap: one pass over
-        field pairs and one over the odd fields (or one over all fields) and the general-column fixup."""
-        nts = [d.shape[0] for d in self.domains]
-        if self.remap_nf == 2:
-            return 8 + any(n >= 2 for n in nts) + any(n % 2 for n in nts) + 1
-        return 8 + 2
+        """Kernel launches of one step (``batch_launches``)."""
+        return batch_launches([d.shape for d in self.domains], self.remap_nf)
 
     def _plan(self, tile_rows: int) -> _Plan:
         if tile_rows not in self._plans:
@@ -223,10 +220,27 @@ class DomainBatch:
                     ms_per_step={f"{k[0]}/{k[1]}": v for k, v in times.items()})
 
 
+def batch_launches(shapes: Sequence[tuple], remap_nf: int) -> int:
+    """Kernel launches of one batched step of domains of these (nt, n, ny, nx) shapes: the FCT passes, one launch each
+    per 64 domains (large batches of one tracer limit in one pass instead of two, ``limit_in_one_pass`` in
+    csrc/advect.cu), then the remap: of a batch that leaves the chip room (``remap_batch_segments`` in csrc/remap.cu) one
+    launch over every field, else one over field pairs and one over the odd fields (or one over all fields) and the
+    general-column fixup."""
+    fct = 0
+    for g in range(0, len(shapes), 64):
+        group = shapes[g:g + 64]
+        one_pass = all(s[0] == 1 for s in group) and sum(s[1] * s[2] * s[3] for s in group) >= 1 << 21
+        fct += FCT_LAUNCHES - one_pass
+    if max(s[1] for s in shapes) <= 96 and sum(s[0] * s[2] * s[3] for s in shapes) <= 150000:
+        return fct + 1
+    if remap_nf == 2:
+        return fct + any(s[0] >= 2 for s in shapes) + any(s[0] % 2 for s in shapes) + 1
+    return fct + 2
+
+
 def sequential_launches(domains: Sequence[Domain]) -> int:
-    """Kernel launches of one ``sequential_step``: 8 FCT passes, then per domain the remap of field pairs (if any),
-    of the odd field (if any) and the general-column fixup."""
-    return sum(8 + (d.shape[0] >= 2) + (d.shape[0] % 2) + 1 for d in domains)
+    """Kernel launches of one ``sequential_step``: per domain the FCT passes and the remap's launches."""
+    return sum(FCT_LAUNCHES + remap_launches(d.shape[0], d.shape[1], d.shape[1]) for d in domains)
 
 
 def sequential_step(domains: Sequence[Domain], parity: int, mixed: bool = False, stream: int | None = None) -> None:

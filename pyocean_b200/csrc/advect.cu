@@ -4,24 +4,27 @@
 // Reference: core/components/tracers.py:208-254, 342-375 and the Numba kernels of
 // core/dynamics/sigma_baroclinic.py:265-364 (faces, RHS), 407-530 (FCT), 856-875 (RK stage).
 //
-// Design.  The reference runs 9 kernels over ~15 full-size temporaries per FCT step.  Here one step is 7 launches:
-//   1-5. for RK stages 1 and 2 a face pass and a cell pass, for stage 3 a face pass (fct_split.cuh): one thread per
-//        cell computes the west x-face and the south y-face of its cell from global memory (L1 serves the
-//        overlapping stencils; no shared memory, no barrier, high occupancy, two independent WENO5 chains per
+// Design.  The reference runs 9 kernels over ~15 full-size temporaries per FCT step.  Here one step is 8 launches:
+//   1.   classes: which reconstruction every face takes, one byte per cell (fct_split.cuh), for all stages and tracers.
+//   2-6. for RK stages 1 and 2 a face pass and a cell pass, for stage 3 a face pass (fct_split.cuh): one thread per
+//        cell computes the west x-face and the south y-face of its cell, of every tracer, from global memory (L1 serves
+//        the overlapping stencils; no shared memory, no barrier, high occupancy, two independent WENO5 chains per
 //        thread), then a streaming pass updates the cells from the stored faces.
 //        1: S <- F0;  c1 = safe(q0 - dt div F0, Va).
 //        2: T <- F1;  q1 recomputed from F0, c2 = safe(3/4 q0 + 1/4 (q1 - dt div F1), Vb).
 //        3: S <- A = ((F0 + F1)/6 + 2 F2/3) - F_L, and c_L = safe(q0 - dt div F_L, V1) from the donor fluxes F_L
 //           of the cell's four faces (recomputed, never stored).
-//   6. coeff  Zalesak R+ / R- per cell from the 7-point (x, y, k +- 1) bounds of C and c_L (tracers looped per
+//   7. coeff  Zalesak R+ / R- per cell from the 7-point (x, y, k +- 1) bounds of C and c_L (tracers looped per
 //             thread: the stencil geometry is read once).
-//   7. final  face coefficients from R of both neighbours; C_out = safe(q0 - dt div(F_L + C A), V1).
+//   8. final  face coefficients from R of both neighbours; C_out = safe(q0 - dt div(F_L + C A), V1).
+// Large batches of one tracer do 7 and 8 in one pass (limit_strip).  The face passes, the coefficient and the final pass
+// leave out the tests for domain edges in the CTAs whose stencils reach none (INNER).
 // The unlimited step (tracers.py:289-291) runs stages 1-2, then a face pass storing the RK3 flux
 // F_H = (F0 + F1)/6 + 2 F2/3 and a cell pass C_out = safe(q0 - dt div F_H, V1).
 // q0 = V0 C, Va, Vb and q1 are recomputed where needed instead of stored.  Planes run k-major (the tracers of one
 // layer follow each other) so a layer's geometry is re-read from L2.  Periodic axes wrap natively in every stencil
 // (the reference pads by TRACER_HALO = 13 cells and crops; with the dependency radius of the step, 10 cells, both
-// give the same numbers).  Workspace: 3 cell stacks (c1 -> R+, c2 -> R-, c_L) and 4 face stacks (S, T).
+// give the same numbers).  Workspace: 3 cell stacks (classes -> R+, c1 -> c_L, c2 -> R-) and 4 face stacks (S, T).
 // An earlier form marched warps along 31-cell strips with a shared-memory row ring and did each stage in one pass;
 // the split form is 14 % faster at 512 x 512 x 50 (the passes are bound by instruction issue and latency, and the
 // simple face threads run at twice the occupancy).
@@ -103,7 +106,9 @@ __device__ __forceinline__ double donor_y(const double* __restrict__ cp, const d
 namespace po {
 
 
-// Pass 4: Zalesak R+ / R- (sigma_baroclinic.py:407-432): bounds over the cell, its x / y neighbours and the layers
+// The limiter: passes 7 and 8.
+//
+// Pass 7: Zalesak R+ / R- (sigma_baroclinic.py:407-432): bounds over the cell, its x / y neighbours and the layers
 // k +- 1 (ok cells), P from the antidiffusive fluxes of the cell's faces, Q from V1 and c_L.  INNER: the CTA's cells have
 // all their x / y neighbours inside the domain.
 template <bool INNER>
@@ -202,7 +207,7 @@ __device__ __forceinline__ double coef_y(const StepArgs& a, const Shape& s, cons
     return A >= 0.0 ? pmin(a.q1[orr], a.c2[ol]) : pmin(a.q1[ol], a.c2[orr]);
 }
 
-// Pass 5: C_out = safe(q0 - dt div(F_L + C A), V1) (sigma_baroclinic.py:514-530).  One thread per column cell
+// Pass 8: C_out = safe(q0 - dt div(F_L + C A), V1) (sigma_baroclinic.py:514-530).  One thread per column cell
 // (k, j, i) loops over the tracers, so the geometry is read once; every value a tracer needs (C, R+ and R- at the
 // cell and its four neighbours, A on the four faces) is loaded before any is used, so the loads of a thread are
 // independent and in flight together.
@@ -293,7 +298,7 @@ __device__ __forceinline__ void final_body(const StepArgs& a, int i0, int j0, in
     else if (i < a.s.nx && j < a.s.ny) final_cell<false>(a, i, j, k);
 }
 
-// Single-domain launches of passes 4 and 5: a 32 x 8 tile of one layer per CTA.
+// Single-domain launches of passes 7 and 8: a 32 x 8 tile of one layer per CTA.
 __global__ void COEFF_BOUNDS fct_coeff_kernel(StepArgs a)
 {
     coeff_body(a, blockIdx.x * TI, blockIdx.y * TJ, a.k0 + blockIdx.z);
@@ -304,7 +309,7 @@ __global__ void FINAL_BOUNDS fct_final_kernel(StepArgs a)
     final_body(a, blockIdx.x * TI, blockIdx.y * TJ, a.k0 + blockIdx.z);
 }
 
-// Batched launches of passes 4 and 5: one 32 x 8 tile of one layer of a domain per CTA.
+// Batched launches of passes 7 and 8: one 32 x 8 tile of one layer of a domain per CTA.
 __global__ void COEFF_BATCHED_BOUNDS fct_coeff_batched(const __grid_constant__ FctBatch B)
 {
     const BlockTile bt = block_tile<false, TI, TJ>(B);
@@ -315,6 +320,168 @@ __global__ void FINAL_BATCHED_BOUNDS fct_final_batched(const __grid_constant__ F
 {
     const BlockTile bt = block_tile<false, TI, TJ>(B);
     final_body(B.a[bt.d], bt.bx * TI, bt.by * TJ, bt.k);
+}
+
+// The limiter pass (sigma_baroclinic.py:407-449, 514-530): Zalesak's R+ / R- of every cell from the 7-point (x, y, k +- 1)
+// bounds of C and c_L and the antidiffusive fluxes A, and from them C_out = safe(q0 - dt div(F_L + C A), V1).
+//
+// A warp takes a strip of 32 cells of one (tracer, layer) plane and marches along j: the bounds' pairs (the larger and
+// smaller of C and c_L of a cell) of rows r-1, r, r+1, R+ / R- of rows r-1, r and the fluxes through the faces between
+// them stay in registers, the neighbours in x come by shuffles, and every face's flux is formed once.  R+ / R- never
+// reach memory and nothing waits at a barrier.  The two outer lanes on either side have no output (their bounds and
+// fluxes lack a neighbour), nor have the two rows before and after a warp's own.
+//
+// Bounded by the latency of its loads (20 warps of 96 registers an SM) and by the 36 % of lanes and rows that only feed
+// others; it saves writing and re-reading R+ and R- and the second read of C, A and the geometry.  24 domains of 96
+// to 384 cells a side, two steps: 16.06 ms with the coefficient and final passes, 15.35 with this one (segments of 32
+// rows 15.37, of 64 15.51; two rows of the march unrolled 15.80, three 16.36; six CTAs an SM 15.65).  With two tracers
+// the two passes read the geometry once for both and are faster (a step at 512 x 512 x 50: 3.45 ms against 3.70), and
+// single domains of one tracer gain 1.4 % at 512 x 512 x 50 but lose 4 to 9 % below 300 x 200 x 30: they keep the passes.
+constexpr int LIMIT_WARPS = 4;                    // warps of a CTA: consecutive row segments of a strip
+constexpr int LIMIT_COLS = 28;                    // cells of a strip that are written
+constexpr int LIMIT_ROWS = 16;                    // rows of a warp's segment
+#define LIMIT_BOUNDS __launch_bounds__(32 * LIMIT_WARPS, 5)
+
+// (max, min) of a cell's C and c_L, first of equals as in the reference's order; neutral for a cell that does not count.
+__device__ __forceinline__ double2 bound_pair(bool counts, double c, double cl)
+{
+    double2 m = make_double2(-INFINITY, INFINITY);
+    m.x = pmax(pmax(m.x, c), cl);
+    m.y = pmin(pmin(m.y, c), cl);
+    return counts ? m : make_double2(-INFINITY, INFINITY);
+}
+
+// F_L + C A of an interior face: the donor value and the limited antidiffusive flux, C = min(R+ downstream, R- upstream)
+// by the sign of A (sigma_baroclinic.py:435-442).  r_l, r_r: (R+, R-) of the cells on its lower and upper side.
+__device__ __forceinline__ double limited_flux(double q, double A, double c_l, double c_r, const double2& r_l,
+                                               const double2& r_r)
+{
+    const double fl = q * (q >= 0 ? c_l : c_r);
+    const double cf = A >= 0.0 ? pmin(r_r.x, r_l.y) : pmin(r_l.x, r_r.y);
+    return fl + cf * A;
+}
+
+// Rows j0 .. j1-1 of the strip whose written cells begin at i0.  INNER: every cell and face within reach of the strip is
+// inside the domain.
+template <bool INNER>
+__device__ __forceinline__ void limit_strip(const StepArgs& a, int t, int k, int i0, int j0, int j1)
+{
+    const Shape s = a.s;
+    const Flags fl(a.flags);
+    const int lane = threadIdx.x & 31;
+    const unsigned all = 0xffffffffu;
+    const bool per_x = !INNER && fl.per_x, per_y = !INNER && fl.per_y;
+    // the lane's cell, on a periodic axis wrapped, else clamped (then the edge's own cell, whose values an edge face
+    // takes); its west face
+    const int ir = i0 - 2 + lane;
+    const int i = INNER ? ir : (per_x ? wrap(ir, s.nx) : min(max(ir, 0), s.nx - 1));
+    const int fx = INNER ? ir : (per_x ? i : min(max(ir, 0), s.nx));
+    const bool in_x = INNER || per_x || (ir >= 0 && ir < s.nx);
+    const bool face_x = INNER || per_x || (ir >= 1 && ir <= s.nx - 1);
+    const bool mine = lane >= 2 && lane < 2 + LIMIT_COLS && ir < s.nx;
+    const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx, p = t * s.n + k;
+    const i64 pc = plane_at(p, pl), gk = plane_at(k, pl);
+    const double* __restrict__ C = a.C + pc;
+    const double* __restrict__ cL = a.c1 + pc;
+    const double* __restrict__ Ax = a.Sx + plane_at(p, xpl);
+    const double* __restrict__ Ay = a.Sy + plane_at(p, ypl);
+    const double* __restrict__ Qx = a.Qx + plane_at(k, xpl);
+    const double* __restrict__ Qy = a.Qy + plane_at(k, ypl);
+    const double* __restrict__ V0 = a.V0 + gk;
+    const double* __restrict__ V1 = a.V1 + gk;
+    const uint8_t* __restrict__ ok = a.ok + gk;
+    double* __restrict__ out = a.out + pc;
+    const int dn = k > 0 ? -pl : 0, up = k + 1 < s.n ? pl : 0;        // the layers below and above
+
+    double2 b_s{0, 0}, b_q{0, 0};           // bounds' pairs of rows q - 1 and q
+    double2 r_s{0, 0};                      // R of row q - 1
+    double c_s = 0.0, c_q = 0.0, l_q = 0.0, a_q = 0.0;
+    double fy_s = 0.0, dx_s = 0.0, v0_s = 0.0, v1_s = 0.0;
+    int o_q = 0, o_s = 0, jq = 0, fq = 0;
+    bool ok_q = false;
+#pragma unroll 1
+    for (int r = j0 - 2; r <= j1 + 1; ++r) {
+        // row r's cells and south faces; row q = r - 1's remaining values
+        const int jr = INNER ? r : (per_y ? wrap(r, s.ny) : min(max(r, 0), s.ny - 1));
+        const int fr = INNER ? r : (per_y ? jr : min(max(r, 0), s.ny));
+        const int o_r = jr * s.nx + i;
+        const double c_r = __ldg(C + o_r), l_r = __ldg(cL + o_r), a_r = __ldg(Ay + (fr * s.nx + i));
+        const bool ok_r = in_x && (INNER || per_y || (r >= 0 && r < s.ny)) && __ldg(ok + o_r) != 0;
+        const int q = r - 1;
+        double2 r_q = make_double2(0.0, 0.0);
+        double fy = 0.0, dx = 0.0, v0 = 0.0, v1 = 0.0;
+        const double2 b_r = bound_pair(ok_r, c_r, l_r);
+        if (r >= j0) {
+            const int oxq = jq * (s.nx + 1) + fx;
+            const double cd = __ldg(C + (o_q + dn)), ld = __ldg(cL + (o_q + dn));
+            const double cu = __ldg(C + (o_q + up)), lu = __ldg(cL + (o_q + up));
+            const bool okd = dn != 0 && __ldg(ok + (o_q + dn)) != 0, oku = up != 0 && __ldg(ok + (o_q + up)) != 0;
+            const double aw = __ldg(Ax + oxq), qw = __ldg(Qx + oxq), qs = __ldg(Qy + (fq * s.nx + i));
+            v1 = __ldg(V1 + o_q);
+            v0 = __ldg(V0 + o_q);
+            const double ae = __shfl_down_sync(all, aw, 1);
+            double2 w, e;
+            w.x = __shfl_up_sync(all, b_q.x, 1);
+            w.y = __shfl_up_sync(all, b_q.y, 1);
+            e.x = __shfl_down_sync(all, b_q.x, 1);
+            e.y = __shfl_down_sync(all, b_q.y, 1);
+            if (ok_q) {
+                const double2 d = bound_pair(okd, cd, ld), u = bound_pair(oku, cu, lu);
+                const double cmax = pmax(pmax(pmax(pmax(pmax(pmax(b_q.x, w.x), e.x), b_s.x), b_r.x), d.x), u.x);
+                const double cmin = pmin(pmin(pmin(pmin(pmin(pmin(b_q.y, w.y), e.y), b_s.y), b_r.y), d.y), u.y);
+                const double p_in = a.dt * (pmax(aw, 0.0) - pmin(ae, 0.0) + pmax(a_q, 0.0) - pmin(a_r, 0.0));
+                const double p_out = a.dt * (pmax(ae, 0.0) - pmin(aw, 0.0) + pmax(a_r, 0.0) - pmin(a_q, 0.0));
+                const double q_in = pmax(v1 * (cmax - l_q), 0.0);
+                const double q_out = pmax(v1 * (l_q - cmin), 0.0);
+                // min(1, q / p): a quotient of q >= p is at least 1, so where the limiter does not bind no division runs
+                if (p_in > 0.0) r_q.x = q_in >= p_in ? 1.0 : pmin(1.0, q_in / p_in);
+                if (p_out > 0.0) r_q.y = q_out >= p_out ? 1.0 : pmin(1.0, q_out / p_out);
+            }
+            // fluxes through row q's west and south faces
+            double2 r_w;
+            r_w.x = __shfl_up_sync(all, r_q.x, 1);
+            r_w.y = __shfl_up_sync(all, r_q.y, 1);
+            const double c_w = __shfl_up_sync(all, c_q, 1);
+            double fw;
+            if (face_x) {
+                fw = limited_flux(qw, aw, c_w, c_q, r_w, r_q);
+            } else {
+                const double ext = a.inflow ? a.inflow[pc + o_q] : c_q;
+                fw = (ir <= 0 ? edge_flux<1>(fl.open_w, qw, c_q, ext) : edge_flux<-1>(fl.open_e, qw, c_q, ext)) + 0.0 * aw;
+            }
+            if (INNER || per_y || (q >= 1 && q <= s.ny - 1)) {
+                fy = limited_flux(qs, a_q, c_s, c_q, r_s, r_q);
+            } else {
+                const double ext = a.inflow ? a.inflow[pc + o_q] : c_q;
+                fy = (q <= 0 ? edge_flux<1>(fl.open_s, qs, c_q, ext) : edge_flux<-1>(fl.open_n, qs, c_q, ext)) + 0.0 * a_q;
+            }
+            dx = __shfl_down_sync(all, fw, 1) - fw;
+        }
+        if (mine && r >= j0 + 2) {                    // row q - 1: its south flux came with the row before
+            const double d = dx_s + fy - fy_s;
+            const double qn = v0_s * c_s - a.dt * d;
+            out[o_s] = v1_s > 0 ? qn / v1_s : c_s;
+        }
+        b_s = b_q; b_q = b_r;
+        r_s = r_q;
+        c_s = c_q; c_q = c_r;
+        l_q = l_r; a_q = a_r;
+        fy_s = fy; dx_s = dx; v0_s = v0; v1_s = v1;
+        o_s = o_q; o_q = o_r;
+        jq = jr; fq = fr;
+        ok_q = ok_r;
+    }
+}
+
+__global__ void LIMIT_BOUNDS fct_limit_batched(const __grid_constant__ FctBatch B)
+{
+    const BlockTile bt = block_tile<true, LIMIT_COLS, LIMIT_ROWS * LIMIT_WARPS>(B);
+    const StepArgs& a = B.a[bt.d];
+    const int i0 = bt.bx * LIMIT_COLS, j0 = (bt.by * LIMIT_WARPS + (threadIdx.x >> 5)) * LIMIT_ROWS;
+    const int j1 = min(j0 + LIMIT_ROWS, a.s.ny);
+    if (j0 >= a.s.ny) return;
+    if (i0 >= 3 && i0 + 30 < a.s.nx && j0 >= 3 && j1 + 2 < a.s.ny) limit_strip<true>(a, bt.t, bt.k, i0, j0, j1);
+    else limit_strip<false>(a, bt.t, bt.k, i0, j0, j1);
 }
 
 // Effective flux F_L + C A of the step through u-face column face_i, (nt, n, ny) (tracers.py:251-254).
@@ -908,6 +1075,14 @@ static void launch_stage(const StepArgs& a, bool mixed, int stage, cudaStream_t 
     else launch_split<false, true>(a, stage, st, nl);
 }
 
+// The limiter's passes over nl layers from a.k0 on.
+static void launch_limit(const StepArgs& a, cudaStream_t st, int nl)
+{
+    const dim3 grid(ceil_div(a.s.nx, TI), ceil_div(a.s.ny, TJ), nl);
+    fct_coeff_kernel<<<grid, NTHREADS, 0, st>>>(a);
+    fct_final_kernel<<<grid, NTHREADS, 0, st>>>(a);
+}
+
 // The FCT step with FP64 (mixed = false) or FP32-weight (mixed = true) WENO faces; everything else FP64.
 static int advect_fct_impl(const char* fn, bool mixed, const double* C, const double* V0, const double* V1,
                            const double* Qx, const double* Qy, const uint8_t* ok, const double* inflow, int nt,
@@ -941,9 +1116,8 @@ static int advect_fct_impl(const char* fn, bool mixed, const double* C, const do
         return pocean_check_launch(fn);
     }
     launch_stage(a, mixed, 3, st, nz);
-    fct_coeff_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nz), NTHREADS, 0, st>>>(a);
-    fct_final_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nz), NTHREADS, 0, st>>>(a);
-    if (fx_face) {
+    launch_limit(a, st, nz);
+    if (fx_face) {          // a kernel of its own: the column's test in the final pass cost that pass 3 % of a large step
         const i64 rows = (i64)nt * nz * ny;
         fct_tef_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(a);
     }
@@ -953,14 +1127,14 @@ static int advect_fct_impl(const char* fn, bool mixed, const double* C, const do
 
 namespace po {
 
-// The CTA ranges of B's domains for a pass over TW x th tiles of their layers, or of their (t, k) planes; returns the
+// The CTA ranges of B's domains for a pass over tw x th tiles of their layers, or of their (t, k) planes; returns the
 // launch's CTAs.
-static unsigned batch_ranges(FctBatch& B, int th, bool planes)
+static unsigned batch_ranges(FctBatch& B, int th, bool planes, int tw = TI)
 {
     int total = 0;
     for (int d = 0; d < B.ndom; ++d) {
         const Shape& s = B.a[d].s;
-        const int tx = ceil_div(s.nx, TI), ty = ceil_div(s.ny, th), count = planes ? s.n * s.nt : s.n;
+        const int tx = ceil_div(s.nx, tw), ty = ceil_div(s.ny, th), count = planes ? s.n * s.nt : s.n;
         B.off[d] = total;
         B.per_layer[d] = tile_magic((long long)tx * ty, count);
         B.per_row[d] = tile_magic(tx, ty);
@@ -985,6 +1159,19 @@ static void fct_batched_stages(FctBatch& B, cudaStream_t st)
     fct_faces3_batched<ZV, MIX, TJR><<<layers, TI * TJR, 0, st>>>(B);
 }
 
+// Whether one marching pass limits a launch's domains instead of the coefficient and the final pass: with one tracer
+// each and enough cells that its long warps fill the chip.  Batches of 0.7 M cells 416 us a step with the two passes, 428
+// with one; 2.6 M 1373 and 1366; 7.9 M 3740 and 3700; 18.9 M 7726 and 7559.
+static bool limit_in_one_pass(const FctBatch& B)
+{
+    i64 cells = 0;
+    for (int d = 0; d < B.ndom; ++d) {
+        if (B.a[d].s.nt > 1) return false;
+        cells += (i64)B.a[d].s.n * B.a[d].s.ny * B.a[d].s.nx;
+    }
+    return cells >= (1ll << 21);
+}
+
 template <bool ZV, bool MIX>
 static void fct_batched_impl(FctBatch& B, int tile_rows, cudaStream_t st)
 {
@@ -993,9 +1180,14 @@ static void fct_batched_impl(FctBatch& B, int tile_rows, cudaStream_t st)
     if (tile_rows == 4) fct_batched_stages<ZV, MIX, 4>(B, st);
     else if (tile_rows == 16) fct_batched_stages<ZV, MIX, 16>(B, st);
     else fct_batched_stages<ZV, MIX, 8>(B, st);
-    const unsigned tiles = batch_ranges(B, TJ, false);
-    fct_coeff_batched<<<tiles, NTHREADS, 0, st>>>(B);
-    fct_final_batched<<<tiles, NTHREADS, 0, st>>>(B);
+    if (!limit_in_one_pass(B)) {
+        const unsigned tiles = batch_ranges(B, TJ, false);
+        fct_coeff_batched<<<tiles, NTHREADS, 0, st>>>(B);
+        fct_final_batched<<<tiles, NTHREADS, 0, st>>>(B);
+        return;
+    }
+    const unsigned strips = batch_ranges(B, LIMIT_ROWS * LIMIT_WARPS, true, LIMIT_COLS);
+    fct_limit_batched<<<strips, 32 * LIMIT_WARPS, 0, st>>>(B);
 }
 
 // The FCT passes of every domain of a batch, one launch per pass and BATCH_CAP domains.
@@ -1233,8 +1425,7 @@ extern "C" int pocean_advect_fct_layers(int mixed, const double* C, const double
         launch_classes(a, st, nl);
         for (int stage = 1; stage <= 3; ++stage) launch_stage(a, mixed != 0, stage, st, nl);
     } else {
-        fct_coeff_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nl), NTHREADS, 0, st>>>(a);
-        fct_final_kernel<<<dim3(ceil_div(nx, TI), ceil_div(ny, TJ), nl), NTHREADS, 0, st>>>(a);
+        launch_limit(a, st, nl);
     }
     return pocean_check_launch(fn);
 }

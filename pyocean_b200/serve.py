@@ -35,7 +35,7 @@ import torch
 
 from . import _lib
 from . import workloads as W
-from .batch import Domain, _Plan, sequential_step
+from .batch import Domain, _Plan, batch_launches, sequential_launches, sequential_step
 
 
 @dataclass
@@ -179,7 +179,7 @@ class Server:
                 for j in step_set:
                     for s in range(k):
                         sequential_step([j.dom], j.flip ^ (s & 1), mixed=self.mixed, stream=stream.cuda_stream)
-                launches += k * sum(8 + (j.nt >= 2) + (j.nt % 2) + 1 for j in step_set)
+                launches += k * sequential_launches([j.dom for j in step_set])
             iters += 1
             occupancy.append(len(step_set))
             done = []
@@ -240,9 +240,7 @@ class Server:
         return chosen
 
     def _launches(self, active) -> int:
-        if self.remap_nf == 2:
-            return 8 + any(j.nt >= 2 for j in active) + any(j.nt % 2 for j in active) + 1
-        return 9
+        return batch_launches([j.dom.shape for j in active], self.remap_nf)
 
     def _retire(self, j: Job, stream) -> None:
         """Marks the job done on the device and releases its buffers (stream-ordered: the caching allocator hands

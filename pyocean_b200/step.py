@@ -14,6 +14,22 @@ import torch
 from . import _lib
 
 
+# Stencil classes, face + cell passes of stages 1 and 2, the stage-3 face pass, limiter coefficients, final update.
+FCT_LAUNCHES = 8
+
+
+def remap_launches(nt: int, n: int, n1: int) -> int:
+    """Kernel launches of a remap of nt fields from n to n1 layers: the field pairs and the single fields, and above 96
+    layers the general-column fixup.  Two fields share a launch where three CTAs' columns fit an SM's shared memory
+    (``segment_smem`` in csrc/remap.cu)."""
+    deep = max(n, n1)
+    if deep > 96:
+        return (nt >= 2) + (nt % 2) + 1
+    pair_bytes = 8 * ((3 * n + n1 + 2 + 2 * (4 * n + 1 + 2 * deep)) * 8 + 2 * n + n1 + 8)
+    pairs = nt // 2 if pair_bytes <= 72 * 1024 else 0
+    return (pairs > 0) + (nt > 2 * pairs)
+
+
 class ALETracerStep:
     """advect_fct + PPM_H4 (or PCM / PLM) remap of a (nt, N, ny, nx) stack with preallocated buffers."""
 
@@ -28,9 +44,7 @@ class ALETracerStep:
         self.ws_bytes = L.pocean_advect_fct_workspace_bytes(nt, n, ny, nx)
         self.ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=self.device)
         self.adv_out = torch.empty((nt, n, ny, nx), dtype=torch.float64, device=self.device)
-        # 8 FCT passes (stencil classes, face + cell for stages 1 and 2, the stage-3 face pass, coefficients, final); the remap:
-        # field pairs (nt >= 2), the odd field (nt odd), the general-column fixup
-        self.launches_per_step = 8 + (nt >= 2) + (nt % 2) + 1
+        self.launches_per_step = FCT_LAUNCHES + remap_launches(nt, n, self.n1)
 
     def stream(self) -> int:
         return torch.cuda.current_stream(self.device).cuda_stream
