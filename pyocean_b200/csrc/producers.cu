@@ -438,8 +438,10 @@ static __device__ __noinline__ void ppm_face_general(const PPMArgs& a, int o, in
 // there.  A face whose correction comes out unchanged stays as it is (its state repeats), so a CTA whose faces are all
 // there leaves its loop.
 //
-// What bounds it: instruction issue in the layers' evaluation, and the sums over the layers, which only other CTAs'
-// work hides (CTAS of them fit an SM): 1.29 ms for 20 steps at 512 x 512 x 50.  As one launch per step, each re-reading
+// What bounds it: latency, with registers and shared memory for 16 warps an SM: the sums over the layers, which only
+// other CTAs' work hides (CTAS of them fit an SM), and the loads of sides that changed (issue slots are 31 % busy).  1.24 ms
+// for 20 steps at 512 x 512 x 50; 1.29 with a test of every layer's velocity for its side in each step and 5 layers a
+// batch of the sums' loads.  As one launch per step, each re-reading
 // 0.63 GB, the 22 passes took 3.55 ms (158 us per step).
 template <int LPT, int W, int CTAS>
 __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int max_iter, int check,
@@ -480,6 +482,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     const double yw = shared_recip(dxw), ye = shared_recip(dxe);
     double edge[LPT], dh[LPT], curv[LPT];
     unsigned west = 0, limited = 0;                // bit l: layer k0 + l holds its west cell's values; has a limit
+    double turn_w = INFINITY, turn_e = -INFINITY;  // the largest -u of the layers on their west side, the smallest on east
 
     // the upwind cell's values of layer k0 + l
     auto load_side = [&](int l, bool w) {
@@ -496,19 +499,18 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     };
     // fluxes and their derivatives of this warp's layers at velocity u (+ du) into shared memory (face_flux)
     auto evaluate = [&](double du, bool shift) {
-        unsigned turned = 0;                       // a velocity whose sign bit is not its side's (-0.0 among them)
-#pragma unroll
-        for (int l = 0; l < LPT; ++l)
-            if (k0 + l < n) {
-                const double v = shift ? shU[(k0 + l) * 32] + du : shU[(k0 + l) * 32];
-                turned |= (((unsigned)__double2hiint(v) >> 31) ^ (west >> l) ^ 1u) & 1u;
-            }
-        if (turned && open) {
+        // u + du >= 0 exactly where du >= -u, so no layer leaves its side while du stays between the sides' bounds
+        if (open && !(du >= turn_w && du < turn_e)) {
+            turn_w = -INFINITY;
+            turn_e = INFINITY;
 #pragma unroll
             for (int l = 0; l < LPT; ++l)
                 if (k0 + l < n) {
-                    const bool w = (shift ? shU[(k0 + l) * 32] + du : shU[(k0 + l) * 32]) >= 0.0;
+                    const double u = shU[(k0 + l) * 32];
+                    const bool w = (shift ? u + du : u) >= 0.0;
                     if (w != (bool)((west >> l) & 1u)) load_side(l, w);
+                    if (w) turn_w = pmax(turn_w, -u);
+                    else turn_e = pmin(turn_e, -u);
                 }
         }
         const unsigned some = __reduce_or_sync(0xffffffffu, limited);
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
             if (k0 + l >= n) break;
             const int r = (k0 + l) * 32;
             const double v = shift ? shU[r] + du : shU[r];
-            const bool w = v >= 0.0;
+            const bool w = (west >> l) & 1u;
             const double c = pmin(quot_rn(fabs(v) * a.dt, w ? dxw : dxe, w ? yw : ye), 1.0);
             double mean = edge[l] + c * (0.5 * dh[l] + curv[l] * (c - 1.5));
             double marg = edge[l] + c * (dh[l] + 3.0 * curv[l] * (c - 1.0));
@@ -586,7 +588,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
         __syncthreads();
         if (wp == 0) {
             double s2 = 0.0, d2 = 0.0;
-#pragma unroll 5
+#pragma unroll 10
             for (int k = 0; k < n; ++k) {
                 s2 += shF[k * 32];
                 d2 += shD[k * 32];
