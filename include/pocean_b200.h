@@ -318,6 +318,16 @@ int pocean_freshwater_volumes_f64(const double* V, const double* dV, const doubl
 int pocean_flux_divergence_f64(const double* Qx, const double* Qy, int nz, int ny, int nx, double* divq,
                                void* stream);
 
+/* What the layer transport leaves of a step, in one pass: h_dag = max(h - dt div Q / A, 0) (as
+ * pocean_flux_divergence_f64 and pocean_lagrangian_thickness_f64, with the same *first_bad), V0 = h A, V1 = h_dag A and
+ * ok = active & V1 > 0. */
+int pocean_layer_state_f64(const double* h, const double* Qx, const double* Qy, const double* area,
+                           const uint8_t* active, int nz, int ny, int nx, double dt, double tol, double* h_dag,
+                           double* V0, double* V1, uint8_t* ok, unsigned long long* first_bad, void* stream);
+
+/* Every plane of a (planes, rows, cols) stack transposed: out is (planes, cols, rows). */
+int pocean_transpose_f64(const double* in, int planes, int rows, int cols, double* out, void* stream);
+
 /* ALE layer volumes V = h A (core/dynamics/sigma_baroclinic.py:1812-1815) and, when ok is not NULL,
  * ok = active & (V > 0) (layer_transport.py:149). */
 int pocean_layer_volumes_f64(const double* h, const double* area, const uint8_t* active, int nz, int ny, int nx,

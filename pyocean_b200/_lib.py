@@ -66,6 +66,8 @@ SIGNATURES: dict[str, tuple] = {
     "pocean_upwind_transport_f64": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _P, _P]),
     "pocean_freshwater_volumes_f64": (_I, [_P, _P, _P, _D, _I, _I, _I, _P, _P, _P]),
     "pocean_flux_divergence_f64": (_I, [_P, _P, _I, _I, _I, _P, _P]),
+    "pocean_layer_state_f64": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _D, _D, _P, _P, _P, _P, _P, _P]),
+    "pocean_transpose_f64": (_I, [_P, _I, _I, _I, _P, _P]),
     "pocean_layer_volumes_f64": (_I, [_P, _P, _P, _I, _I, _I, _P, _P, _P]),
     "pocean_regrid_columns_f64": (_I, [_I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _D, _D, _D, _I, _I, _I, _I, _I, _P,
                                        _P]),

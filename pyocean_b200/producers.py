@@ -178,7 +178,14 @@ class LayerFluxes:
 
 
 def _swap(t: torch.Tensor) -> torch.Tensor:
-    return t.transpose(-1, -2).contiguous()
+    """``t`` with its last two axes exchanged, contiguous."""
+    if not (t.is_cuda and t.dtype == torch.float64 and t.is_contiguous() and t.numel() and max(t.shape) < 2 ** 31):
+        return t.transpose(-1, -2).contiguous()
+    rows, cols = t.shape[-2:]
+    out = torch.empty((*t.shape[:-2], cols, rows), dtype=t.dtype, device=t.device)
+    _lib.check(_lib.lib().pocean_transpose_f64(t.data_ptr(), t.numel() // (rows * cols), rows, cols, out.data_ptr(),
+                                               torch.cuda.current_stream(t.device).cuda_stream), "transpose")
+    return out
 
 
 PPM_HALO = 4                           # core/components/layer_transport.py:122 (the PPM edges' stencil)
@@ -315,16 +322,18 @@ class ALELayerTransport:
                                  cv.f64(fluxes.open_Qu, (ny, nx + 1)), cv.f64(fluxes.open_Qv, (ny + 1, nx)),
                                  cv.f64(fs.Lu, (ny, nx + 1)), cv.f64(fs.Lv, (ny + 1, nx)), tb)
         Qx, Qy, n_lim = limit_outflow(h, Qx, Qy, area, dt, act, periodic=(px, py))
-        divh = cv.empty((n, ny, nx))
-        _lib.check(L.pocean_flux_divergence_f64(Qx.data_ptr(), Qy.data_ptr(), n, ny, nx, divh.data_ptr(),
-                                                cv.stream()), "flux_divergence")
-        h_lag = lagrangian_thickness(h, divh, dt, area)
-        V0, V1 = cv.empty((n, ny, nx)), cv.empty((n, ny, nx))
+        h_lag, V0, V1 = cv.empty((n, ny, nx)), cv.empty((n, ny, nx)), cv.empty((n, ny, nx))
         ok = torch.empty((n, ny, nx), dtype=torch.uint8, device=cv.device)
-        for hh, V, o in ((h, V0, None), (h_lag, V1, ok)):
-            _lib.check(L.pocean_layer_volumes_f64(hh.data_ptr(), area.data_ptr(), act.data_ptr(), n, ny, nx,
-                                                  V.data_ptr(), None if o is None else o.data_ptr(), cv.stream()),
-                       "layer_volumes")
+        bad = torch.empty(1, dtype=torch.int64, device=cv.device)
+        _lib.check(L.pocean_layer_state_f64(h.data_ptr(), Qx.data_ptr(), Qy.data_ptr(), area.data_ptr(),
+                                            act.data_ptr(), n, ny, nx, float(dt), 1e-9, h_lag.data_ptr(),
+                                            V0.data_ptr(), V1.data_ptr(), ok.data_ptr(), bad.data_ptr(),
+                                            cv.stream()), "layer_state")
+        if int(bad.item()) != -1:                      # a layer emptied: lagrangian_thickness names it and raises
+            divh = cv.empty((n, ny, nx))
+            _lib.check(L.pocean_flux_divergence_f64(Qx.data_ptr(), Qy.data_ptr(), n, ny, nx, divh.data_ptr(),
+                                                    cv.stream()), "flux_divergence")
+            lagrangian_thickness(h, divh, dt, area)
         Fz = torch.zeros((n + 1, ny, nx), dtype=torch.float64, device=cv.device)
         h_fw = V_fw = None
         if fw is not None:
@@ -332,7 +341,7 @@ class ALELayerTransport:
             V_fw = cv.empty((n, ny, nx))
             _lib.check(L.pocean_layer_volumes_f64(h_fw.data_ptr(), area.data_ptr(), act.data_ptr(), n, ny, nx,
                                                   V_fw.data_ptr(), None, cv.stream()), "layer_volumes")
-        okb = ok.bool()
+        okb = ok.view(torch.bool)                      # written as 0 / 1
         return LayerFluxes(cv.out(Qx), cv.out(Qy), cv.out(Fz), cv.out(V0), cv.out(V1),
                            okb.cpu().numpy() if cv.numpy_out else okb, cv.out(h_lag), int(n_lim),
                            None if V_fw is None else cv.out(V_fw), None if h_fw is None else cv.out(h_fw))
