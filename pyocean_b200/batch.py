@@ -2,7 +2,7 @@
 Batched ALE tracer steps of many independent, unevenly sized domains on one GPU.
 
 One step of every domain is ``advect_fct`` of its stack followed by the remap of every stack member onto its target
-grid (the reference's phases 7 and 8, core/model/driver.py:888-985, run once per domain).  Instead of 10-11 kernel
+grid (the reference's phases 7 and 8, core/model/driver.py:888-985, run once per domain).  Instead of 9-10 kernel
 launches per domain and step, each pass of the step is ONE launch over all domains: the CTAs of a launch are split
 into per-domain ranges by a CTA-offset table and every CTA finds its domain by binary search, so small domains share
 the GPU instead of each leaving most of the 148 SMs idle.  A step sequence only enqueues kernels and is captured in
@@ -244,7 +244,7 @@ def sequential_launches(domains: Sequence[Domain]) -> int:
 
 
 def sequential_step(domains: Sequence[Domain], parity: int, mixed: bool = False, stream: int | None = None) -> None:
-    """One step of every domain with the single-domain entry points, one domain after another (7-8 plain launches
+    """One step of every domain with the single-domain entry points, one domain after another (9-10 plain launches
     per domain), on the same buffers as the batch: the form a batch replaces."""
     L = _lib.lib()
     fn = L.pocean_advect_fct_mixed if mixed else L.pocean_advect_fct_f64

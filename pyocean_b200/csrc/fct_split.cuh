@@ -1,9 +1,9 @@
 // The three WENO passes of the FCT step split into a face pass and a cell pass each (included by advect.cu).
 //
-// Face pass of stage s: one thread per cell (t, k, j, i) computes the west x-face and the south y-face of its cell
-// (the last column / row also the east / north domain face) straight from global memory (the five upwind cells of
-// a face, loaded in upwind order, overlap between neighbouring threads and are served by L1), with no shared memory
-// and no barrier, so the pass runs
+// Face pass of stage s: one thread per cell (k, j, i), every tracer in turn, computes the west x-face and the south y-face
+// of its cell (the last column / row also the east / north domain face) straight from global memory (the five upwind
+// cells of a face, loaded in upwind order, overlap between neighbouring threads and are served by L1), with no shared
+// memory and no barrier, so the pass runs
 // at high occupancy and the two independent WENO5 chains of a thread overlap.  Cell pass of stage s: the stage
 // update from the stored faces.  Faces per stage are stored once:
 //   stage 1: S <- F0;  stage 2: T <- F1;  stage 3: S <- A = ((F0 + F1)/6 + 2 F2/3) - F_L,
@@ -11,9 +11,8 @@
 // face pass also forms the donor-cell solution c_L of its cell, recomputing the cheap donor fluxes F_L of the
 // cell's east and north faces, so F_L is never stored.  The arithmetic of every face and
 // update is the reference's (weno.cuh; sigma_baroclinic.py:265-321, 452-511), so results equal the reference's bit
-// for bit.  Addresses are formed once per thread as plane pointers with 32-bit offsets; interior stencils (all six
-// candidate cells inside the domain, the common case) load without checks, edge and periodic stencils take a guarded
-// path.
+// for bit.  Which reconstruction a face takes comes from the class pass; CTAs
+// whose stencils stay inside the domain run without the edge and periodic cases (INNER).
 #pragma once
 
 namespace po {
