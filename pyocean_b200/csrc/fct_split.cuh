@@ -56,12 +56,23 @@ __device__ __forceinline__ unsigned line_class(const uint8_t* __restrict__ ok, i
 }
 
 // Validity of four neighbouring cells as the bytes of a word (0xff valid, 0 not): cells i .. i+3 of a row of n cells,
-// 0 outside the row (a periodic row wraps).  `row4` is the row's word when its cells may be read four at a time.
-__device__ __forceinline__ unsigned ok4(const uint8_t* __restrict__ row, int n, bool per, int i, bool words)
+// 0 outside the row (a periodic row wraps); i is a multiple of four.  `words`: rows start on words.  Other rows are read
+// as the two words around the cells where both lie within the mask (lo .. hi), the cells beyond the row cleared; what is
+// left (the wrapped ends, the mask's own ends) goes by bytes.
+__device__ __forceinline__ unsigned ok4(const uint8_t* __restrict__ row, int n, bool per, int i, bool words,
+                                        const uint8_t* lo, const uint8_t* hi)
 {
+    if (!per && (i < 0 || i >= n)) return 0u;
     unsigned w = 0;
+    const uint8_t* p = row + i;
+    const unsigned off = (unsigned)reinterpret_cast<uintptr_t>(p) & 3u;
+    const uint8_t* q = p - off;
     if (words && i >= 0 && i + 4 <= n) {
-        w = __ldg(reinterpret_cast<const unsigned*>(row + i));
+        w = __ldg(reinterpret_cast<const unsigned*>(p));
+    } else if (i >= 0 && (i + 4 <= n || !per) && q >= lo && q + 8 <= hi) {
+        const unsigned* q4 = reinterpret_cast<const unsigned*>(q);
+        w = __funnelshift_r(__ldg(q4), __ldg(q4 + 1), 8 * off);
+        if (i + 4 > n) w &= (1u << (8 * (n - i))) - 1u;
     } else {
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -94,8 +105,9 @@ __device__ __forceinline__ void class_body(const StepArgs& a, int k, int i, int 
     const uint8_t* ok = a.ok + plane_at(k, pl);
     const bool words = (s.nx & 3) == 0 && (reinterpret_cast<uintptr_t>(ok) & 3) == 0;
     const uint8_t* row = ok + j * s.nx;
-    const unsigned w0 = ok4(row, s.nx, fl.per_x, i - 4, words), w1 = ok4(row, s.nx, fl.per_x, i, words),
-                   w2 = ok4(row, s.nx, fl.per_x, i + 4, words);
+    const uint8_t *lo = a.ok, *hi = a.ok + plane_at(s.n, pl);
+    const unsigned w0 = ok4(row, s.nx, fl.per_x, i - 4, words, lo, hi), w1 = ok4(row, s.nx, fl.per_x, i, words, lo, hi),
+                   w2 = ok4(row, s.nx, fl.per_x, i + 4, words, lo, hi);
     unsigned v[6];
     v[0] = __funnelshift_r(w0, w1, 8);                                        // cells i-3 .. i
     v[1] = __funnelshift_r(w0, w1, 16);
@@ -108,7 +120,7 @@ __device__ __forceinline__ void class_body(const StepArgs& a, int k, int i, int 
     for (int m = 0; m < 6; ++m) {
         int g = j - 3 + m;
         if (fl.per_y) g = wrap(g, s.ny);
-        v[m] = m == 3 ? w1 : (g >= 0 && g < s.ny ? ok4(ok + g * s.nx, s.nx, false, i, words) : 0u);
+        v[m] = m == 3 ? w1 : (g >= 0 && g < s.ny ? ok4(ok + g * s.nx, s.nx, false, i, words, lo, hi) : 0u);
     }
     c |= class4(v) << 4;
     uint8_t* out = fct_classes(a) + plane_at(k, pl) + (j * s.nx + i);
