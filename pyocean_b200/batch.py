@@ -240,7 +240,7 @@ def batch_launches(shapes: Sequence[tuple], remap_nf: int) -> int:
 
 def sequential_launches(domains: Sequence[Domain]) -> int:
     """Kernel launches of one ``sequential_step``: per domain the FCT passes and the remap's launches."""
-    return sum(FCT_LAUNCHES + remap_launches(d.shape[0], d.shape[1], d.shape[1]) for d in domains)
+    return sum(FCT_LAUNCHES + remap_launches(d.shape[0], d.shape[1], d.shape[1], d.shape[2] * d.shape[3]) for d in domains)
 
 
 def sequential_step(domains: Sequence[Domain], parity: int, mixed: bool = False, stream: int | None = None) -> None:

@@ -78,3 +78,13 @@ def test_batched_columns_of_different_depths(nf_mode, deep):
         adv.per = P.Periodic(w.periodic)
         ref = P.remap_columns(w.h_src, adv.advect_fct(w.C, w.V0, w.V1, w.Qx, w.Qy, w.ok), w.h_tgt, w.remap_scheme, w.wet)
         np.testing.assert_array_equal(batch.state(i).cpu().numpy(), ref)
+
+
+def test_deep_pairs_of_a_large_plane():
+    """Deep field pairs of a plane that fills the chip go by the sweep, single fields layer by layer: same values."""
+    import torch
+    hs, f, ht, wet = (torch.from_numpy(x).cuda() for x in _columns(17, 75, 75, 388, 389, 3))
+    got = P.remap_columns(hs, f, ht, P.PPM_H4, wet)
+    for m in range(3):
+        one = P.remap_columns(hs, f[m:m + 1].contiguous(), ht, P.PPM_H4, wet)
+        assert torch.equal(got[m].view(torch.int64), one[0].view(torch.int64))
