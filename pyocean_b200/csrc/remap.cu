@@ -569,10 +569,10 @@ bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::S
 // Columns of a batched remap CTA.
 int remap_batched_columns(bool segments) { return segments ? remap::SG_BATCH_COLS : 128; }
 
-// Dynamic shared memory above the default limit has to be asked for.
+// A kernel's static and dynamic shared memory together above the default limit (48 KB) has to be asked for; the static part
+// is the compiler's, so every size asks.
 static cudaError_t allow_smem(const void* kernel, size_t bytes)
 {
-    if (bytes <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
