@@ -569,11 +569,16 @@ bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::S
 // Columns of a batched remap CTA.
 int remap_batched_columns(bool segments) { return segments ? remap::SG_BATCH_COLS : 128; }
 
-// A kernel's static and dynamic shared memory together above the default limit (48 KB) has to be asked for; the static part
-// is the compiler's, so every size asks.
-static cudaError_t allow_smem(const void* kernel, size_t bytes)
+// The most dynamic shared memory a side-by-side launch takes: columns of SG_LAYERS layers of one field; field pairs up to
+// three CTAs an SM.
+constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_LAYERS), SG_SMEM2 = 72 * 1024;
+
+// A kernel's static and dynamic shared memory together above the default limit (48 KB) has to be asked for.  The limit
+// belongs to the kernel, not to the launch: every call asks for the same, so that no other thread's call lowers it between
+// a call's request and its launch.
+static cudaError_t allow_smem(const void* kernel, size_t most)
 {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 // nf_mode 2: field pairs (+ the odd field); nf_mode 1: every field on its own.  nmax: the batch's deepest column.
@@ -584,7 +589,7 @@ cudaError_t remap_batched_launch(const BatchDomain* doms, const int* off_dev, co
     auto offs = [&](int pass) { return off_dev + pass * (ndom + 1); };
     if (segments) {
         const size_t smem = remap::segment_smem(1, nmax, nmax);
-        const cudaError_t e = allow_smem((const void*)remap::remap_segments_batched, smem);
+        const cudaError_t e = allow_smem((const void*)remap::remap_segments_batched, SG_SMEM1);
         if (e != cudaSuccess) return e;
         remap::remap_segments_batched<<<total(BP_RALL), remap::SG_THREADS, smem, st>>>(doms, offs(BP_RALL), ndom);
         return cudaSuccess;
@@ -637,7 +642,7 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
     // Side by side, two fields of a column share the work on its thicknesses while three CTAs fit an SM.  Where they do not
     // (above 70 layers) and the columns fill the chip, the sweep's field pairs are faster: two fields of 512 x 512 x 75
     // take 0.79 ms as two single fields side by side, 0.62 by the sweep; 60 x 60 x 75 with four 24 us against 176.
-    const bool fit2 = remap::segment_smem(2, n0, n1) <= 72 * 1024;
+    const bool fit2 = remap::segment_smem(2, n0, n1) <= SG_SMEM2;
     if ((n0 > n1 ? n0 : n1) <= remap::SG_LAYERS && (fit2 || nfields == 1 || plane < 150000)) {
         const int nf2 = fit2 ? nfields / 2 : 0, rest = nfields - 2 * nf2;
         const int threads = remap::segment_threads(n0, n1);
@@ -645,8 +650,8 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
         const size_t s1 = remap::segment_smem(1, n0, n1), s2 = remap::segment_smem(2, n0, n1);
         const auto one = s1 <= remap::SG_FIVE ? remap::remap_segments_kernel<1, 5> : remap::remap_segments_kernel<1, 4>;
         const auto two = remap::remap_segments_kernel<2, 4>;
-        cudaError_t e = rest ? allow_smem((const void*)one, s1) : cudaSuccess;
-        if (e == cudaSuccess && nf2) e = allow_smem((const void*)two, s2);
+        cudaError_t e = rest ? allow_smem((const void*)one, SG_SMEM1) : cudaSuccess;
+        if (e == cudaSuccess && nf2) e = allow_smem((const void*)two, SG_SMEM2);
         if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
         if (nf2) two<<<g, threads, s2, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 0, scheme, out);
         if (rest)

@@ -31,3 +31,34 @@ def test_depths_between_the_dynamic_and_the_whole_limit():
     r = subprocess.run([sys.executable, "-c", CHECK], cwd=ROOT, capture_output=True, text=True, timeout=300,
                        env={**os.environ, "PYTHONPATH": ROOT})
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_two_depths_from_several_threads():
+    """A launch never meets the limit of another thread's depth."""
+    import threading
+
+    import torch
+
+    from pyocean_b200 import _lib
+    dev, fn, bad = torch.device("cuda", 0), _lib.lib().pocean_remap_columns_f64, []
+    go = threading.Barrier(8)
+
+    def work(n):
+        h = torch.full((n, 4, 4), 2.0, device=dev, dtype=torch.float64)
+        f, w = torch.rand_like(h), torch.ones((4, 4), device=dev, dtype=torch.uint8)
+        o, s = torch.empty_like(h), torch.cuda.Stream(dev)
+        s.wait_stream(torch.cuda.current_stream(dev))
+        go.wait()
+        bad.extend(rc for rc in (fn(h.data_ptr(), f.data_ptr(), h.data_ptr(), w.data_ptr(), n, n, 4, 4, 1, 2,
+                                    o.data_ptr(), s.cuda_stream) for _ in range(4000)) if rc)
+        s.synchronize()
+        if not torch.allclose(o, f, rtol=1e-12, atol=0.0):        # the same grid: the field, but for rounding
+            bad.append(f"depth {n}: wrong values")
+
+    threads = [threading.Thread(target=work, args=((76, 96)[i % 2],)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize(dev)
+    assert not bad, (len(bad), bad[:3])
