@@ -96,21 +96,6 @@ struct FctBatch {
 };
 static_assert(sizeof(FctBatch) <= 32000, "kernel parameters hold 32764 bytes");
 
-// x / d for 0 <= x < d count as a multiply: with m = ceil(2^47 / d), e = m d - 2^47 < d, floor(x m / 2^47) = x / d
-// whenever x e < 2^47 (Granlund & Montgomery 1994), which d d count < 2^47 ensures, and x m < 2^47 count fits 64 bits
-// (count <= 65535).  Else 0: the division itself.
-inline unsigned long long tile_magic(long long d, long long count)
-{
-    constexpr unsigned long long one = 1ull << 47;
-    if ((double)d * (double)d * (double)count >= 1.4e14) return 0ull;
-    return (one + (unsigned long long)d - 1) / (unsigned long long)d;
-}
-
-__device__ __forceinline__ int tile_div(int x, unsigned long long m, int d)
-{
-    return m ? (int)(((unsigned long long)(unsigned)x * m) >> 47) : x / d;
-}
-
 // The FCT workspace cut into a's buffers (advect.cu).
 void carve_fct_workspace(StepArgs& a, void* workspace);
 
