@@ -1,5 +1,5 @@
 // Correctly rounded division of binary64 values by the constants 3 and 6 in three FP64 operations, and by a divisor
-// whose correctly rounded reciprocal is at hand.
+// whose reciprocal is at hand.
 //
 // The reference divides by 6 three times per WENO face ((2v1 - 7v2 + 11v3)/6 ...) and by 3 in the RK3 flux
 // combination.  An IEEE division is an iterative sequence of ~10 FP64 instructions; for these constant divisors
@@ -79,39 +79,45 @@ PO_XD double div6_exact(double x)
 }
 
 #ifdef __CUDACC__
-// RN(1 / b) for 2^-1000 < b < 2^1000 without range checks: the hardware's approximate reciprocal (relative error e
-// about 2^-20: it reads the upper 20 mantissa bits of b and gives as many), one cubic step y (1 + e + e^2), which leaves
-// e^3 and the rounding (below one ulp), and Markstein's final step, after which y is the correctly rounded reciprocal
-// unless b's mantissa is all ones and y came out below (P. Markstein, "IA-64 and Elementary Functions", 2000, ch. 8).
-// For that mantissa 1 / b lies just above the middle of two doubles; the bit set below the approximation's last one
-// makes it an overestimate there, e^3 negative, and y the upper neighbour, which the final step keeps.
-__device__ __forceinline__ double recip_rn(double b)
+// 1 / b for 2^-1000 < b < 2^1000 without range checks, for quot_rn: PTX's approximate reciprocal (rcp.approx.ftz.f64: it
+// reads the upper 20 mantissa bits of b and gives as many; relative error e below 2^-18) and two Newton-Raphson steps
+// y (1 + e) (P. Markstein, "IA-64 and Elementary Functions", 2000, ch. 8).  A step squares the relative error, so the
+// result lies within 2^-72 of 1 / b before its own rounding: within (1/2 + eta) ulp with eta = 2^-19.
+__device__ __forceinline__ double recip_newton(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = __hiloint2double(__double2hiint(y), (int)0x80000000);
-    double e = fma(-b, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
-    e = fma(-b, y, 1.0);
-    return fma(y, e, y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
 }
 
-// RN(a / b), b > 0, from y = RN(1 / b) (the same chapter: the quotient a y is within one ulp, its residual is exact and
-// one correction rounds correctly), for quotients and residuals that stay normal: |a| >= 2^-960, |a / b| in
-// [2^-1000, 2^1000]; or a = +-0, whose sign the residual's order keeps.
+// RN(a / b), b > 0, for quotients and residuals that stay normal: |a| >= 2^-960, |a / b| in [2^-1000, 2^1000]; or a = +-0,
+// whose sign the residual's order keeps.  y: RN(1 / b), or recip_newton(b) where b is not near_two.
+//
+// One correction of q = RN(a y) by its exact residual r = a - b q (Markstein's, the same chapter): q + r y differs from
+// a / b by (r / b)(b y - 1).  Scaled to b in [1, 2), a / b in [1, 2): a / b is no midpoint of two doubles and lies at least
+// 2^-105 / b from the nearest, M.  Only a distance below 2^-100 can matter (the difference is smaller than that); then
+// |a / b - q| is half an ulp, 2^-53 (three halves would take |a y - a / b| of an ulp, so b > 2 (1 - 2 eta)), and with
+// |b y - 1| <= b (1 + 2 eta) 2^-54 the difference is at most b (1 + 2 eta) 2^-107, less than 2^-105 / b where
+// b^2 (1 + 2 eta) < 4: for every b with eta = 0, else for b < 2 - 2^-18.
 __device__ __forceinline__ double quot_rn(double a, double b, double y)
 {
     const double q = a * y;
     return fma(fma(b, q, -a), -y, q);
 }
 
-// Divisors shared by several quotients: y = RN(1 / b) once, three operations per quotient; 0 for a b outside
-// [2^-400, 2^400].  quotient(a, b, y) is a / b; it takes the division for y = 0 and for an a that is neither 0 nor in
-// [2^-500, 2^500].
+// Whether recip_newton(b) may not serve quot_rn: the upper 18 mantissa bits of b are ones.  near_two_bits of several
+// divisors can be compared by their maximum.
+__device__ __forceinline__ unsigned near_two_bits(double b) { return (unsigned)__double2hiint(b) << 12; }
+constexpr unsigned NEAR_TWO = 0xffffc000u;
+
+// Divisors shared by several quotients: y = 1 / b once, three operations per quotient; 0 for a b outside
+// [2^-400, 2^400] or near two.  quotient(a, b, y) is a / b; it takes the division for y = 0 and for an a that is neither 0
+// nor in [2^-500, 2^500].
 __device__ __forceinline__ double shared_recip(double b)
 {
     const bool in = (unsigned)__double2hiint(b) - (623u << 20) < (800u << 20);         // b > 0 too
-    return in ? recip_rn(b) : 0.0;
+    return in && near_two_bits(b) < NEAR_TWO ? recip_newton(b) : 0.0;
 }
 
 __device__ __forceinline__ double quotient(double a, double b, double y)

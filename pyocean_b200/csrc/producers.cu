@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     const int k0 = wp * LPT;
     // a closed face: width 1, velocity, edges and length 0, so that its fluxes come out +0
     const double dxw = open ? fc.dxw : 1.0, dxe = open ? fc.dxe : 1.0, L_f = open ? __ldg(a.L + oc) : 0.0;
-    const double yw = shared_recip(dxw), ye = shared_recip(dxe);
+    const double yw = 1.0 / dxw, ye = 1.0 / dxe;
     double edge[LPT], dh[LPT], curv[LPT];
     unsigned west = 0, limited = 0;                // bit l: layer k0 + l holds its west cell's values; has a limit
     double turn_w = INFINITY, turn_e = -INFINITY;  // the largest -u of the layers on their west side, the smallest on east
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     auto mid = [](double x) {                      // |x| in [2^-250, 2^250): no quotient below leaves the range
         return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (773u << 20) < (500u << 20);
     };
-    bool odd = open && !(mid(dxw) && mid(dxe) && mid(a.dt) && yw != 0.0 && ye != 0.0 && a.dt > 0.0);
+    bool odd = open && !(mid(dxw) && mid(dxe) && mid(a.dt) && dxw > 0.0 && dxe > 0.0 && a.dt > 0.0);
 #pragma unroll
     for (int l = 0; l < LPT; ++l) {
         edge[l] = dh[l] = curv[l] = 0.0;

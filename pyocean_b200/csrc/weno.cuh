@@ -55,16 +55,17 @@ static __constant__ double kWeno[6] = {13.0 / 12.0, 1e-40, 1e-6, 0.1, 0.6, 0.3};
 // WENO5 value of a stencil whose five cells are valid: the numbers of weno5_ieee in fewer instructions.
 //  * A product by a power of two is exact, so a - 2 b, a - 4 b and a + 0.25 b are one fma each with the same rounding
 //    (0.25 (e e) may round in the subnormal range; beside the epsilon 1e-40 or 1e-6 that changes no bit).
-//  * A face costs 77 FP64 instructions and about as many others; with four IEEE divisions and their checks it cost 92
+//  * A face costs 73 FP64 instructions and about as many others; with four IEEE divisions and their checks it cost 92
 //    and 225 (ncu, face pass of 384 x 384 x 50, T and S: 634 -> 379 warp instructions per warp of 64 faces with the
 //    stencil classes, 317 -> 242 us).
 //  * x / 6 takes three operations (div6_short), the four quotients a reciprocal and one correction each
-//    (recip_rn, quot_rn), without range checks of their own.
+//    (recip_newton, quot_rn), without range checks of their own.
 //  * One check per face covers all of them.  The weights' denominators are below 2^800 (JS: their roots below 2^50):
 //    with the epsilon below them, the reciprocals and quotients are normal numbers, and a quotient too small for an
 //    exact residual is added to 1 and vanishes.  The face value is in [2^-800, 2^900): then the last residual is exact,
 //    no term was infinite or NaN, and a candidate x / 6 below 2^-1019, which div6_short may round differently, is too
-//    small against the others to be seen.  Anything else, and the value 0, goes to weno5_ieee.
+//    small against the others to be seen.  No divisor is near two (four of 2^18 faces have one).  Anything else, and the
+//    value 0, goes to weno5_ieee.
 template <bool ZV>
 __device__ __forceinline__ double weno5_full(double v1, double v2, double v3, double v4, double v5)
 {
@@ -85,24 +86,28 @@ __device__ __forceinline__ double weno5_full(double v1, double v2, double v3, do
     const double g0 = eps + b0, g1 = eps + b1, g2 = eps + b2;
     const unsigned top = max(max((unsigned)__double2hiint(g0), (unsigned)__double2hiint(g1)),
                              (unsigned)__double2hiint(g2));
+    constexpr unsigned lim = (1023u + (ZV ? 800u : 50u)) << 20;
+    // the divisors of the three weights; their checks first, so that no bits of them stay in registers for the end (kept
+    // there they cost a step at 512 x 512 x 50 1.5 % in spills)
+    const double s0 = ZV ? g0 : g0 * g0, s1 = ZV ? g1 : g1 * g1, s2 = ZV ? g2 : g2 * g2;
+    bool slow = max(max(near_two_bits(s0), near_two_bits(s1)), near_two_bits(s2)) >= NEAR_TWO || top >= lim;
     double a0, a1, a2;
     if (ZV) {
         const double tau = fabs(b2 - b0);
-        a0 = kWeno[3] * (1.0 + quot_rn(tau, g0, recip_rn(g0)));
-        a1 = kWeno[4] * (1.0 + quot_rn(tau, g1, recip_rn(g1)));
-        a2 = kWeno[5] * (1.0 + quot_rn(tau, g2, recip_rn(g2)));
+        a0 = kWeno[3] * (1.0 + quot_rn(tau, s0, recip_newton(s0)));
+        a1 = kWeno[4] * (1.0 + quot_rn(tau, s1, recip_newton(s1)));
+        a2 = kWeno[5] * (1.0 + quot_rn(tau, s2, recip_newton(s2)));
     } else {
-        const double s0 = g0 * g0, s1 = g1 * g1, s2 = g2 * g2;
-        a0 = quot_rn(kWeno[3], s0, recip_rn(s0));
-        a1 = quot_rn(kWeno[4], s1, recip_rn(s1));
-        a2 = quot_rn(kWeno[5], s2, recip_rn(s2));
+        a0 = quot_rn(kWeno[3], s0, recip_newton(s0));
+        a1 = quot_rn(kWeno[4], s1, recip_newton(s1));
+        a2 = quot_rn(kWeno[5], s2, recip_newton(s2));
     }
     const double den = a0 + a1 + a2;
-    const double w = quot_rn(a0 * q0 + a1 * q1 + a2 * q2, den, recip_rn(den));
+    slow = slow || near_two_bits(den) >= NEAR_TWO;
+    const double w = quot_rn(a0 * q0 + a1 * q1 + a2 * q2, den, recip_newton(den));
     const unsigned size = (unsigned)__double2hiint(w) & 0x7fffffffu;
     constexpr unsigned lo = (1023u - 800u) << 20, hi = (1023u + 900u) << 20;
-    constexpr unsigned lim = (1023u + (ZV ? 800u : 50u)) << 20;
-    if (size - lo >= hi - lo || top >= lim) return weno5_ieee(v1, v2, v3, v4, v5, ZV);
+    if (size - lo >= hi - lo || slow) return weno5_ieee(v1, v2, v3, v4, v5, ZV);
     return w;
 }
 
