@@ -58,25 +58,32 @@ def test_ordinary_numbers(check, seed):
     check(a, np.resize(_divisors(rng, 1 << 20), a.size))
 
 
-def test_quotients_next_to_the_middle_of_two_doubles(check):
-    """a / b = (2 N + 1) / 2 ulp +- k / B: for odd B, A 2^53 = +-k (mod B)."""
-    rng = np.random.default_rng(5)
-    near = [(1 << 53) - k for k in range(1, 4000, 2)]
-    limit = [(1 << 53) - (1 << 34) + d for d in range(-3999, 4000, 2)]
-    some = [int(x) | 1 for x in rng.integers(1 << 52, 1 << 53, 6000)]
+def _next_to_midpoints(divisors):
+    """53-bit integers A for each odd 53-bit B with A / B next to the middle of two doubles: A 2^e = N B + k, N odd of 54 bits
+    (e = 53 for A > B, 54 for A < B), k small."""
     a, b = [], []
-    for B in near + limit + some:
-        inv = pow(1 << 53, -1, B)
-        for k in (1, 2, 3, 5, -1, -2, -3, -5):
-            A = k * inv % B
-            for cand in (A, A + B, 2 * A, 2 * (A + B)):
-                while 0 < cand < 1 << 52:
-                    cand *= 2
-                if 1 << 52 <= cand < 1 << 53:
-                    a.append(float(cand))
+    for B in divisors:
+        for e in (53, 54):
+            inv = pow(1 << e, -1, B)
+            for k in (1, 2, 3, 5, 9, -1, -2, -3, -5, -9):
+                A = k * inv % B
+                A += B if e == 53 else 0
+                N = ((A << e) - k) // B
+                if 1 << 52 <= A < 1 << 53 and 1 << 53 <= N < 1 << 54 and N & 1:
+                    a.append(float(A))
                     b.append(float(B))
-    assert len(a) > 50000
-    check(a, b)
+    return a, b
+
+
+def test_quotients_next_to_the_middle_of_two_doubles(check):
+    rng = np.random.default_rng(5)
+    near = [(1 << 53) - k for k in range(1, 20000, 2)]
+    limit = [(1 << 53) - (1 << 34) + d for d in range(-9999, 10000, 2)]
+    some = [int(x) | 1 for x in rng.integers(1 << 52, 1 << 53, 20000)]
+    for divisors in (near, limit, some):
+        a, b = _next_to_midpoints(divisors)
+        assert len(a) > 20000
+        check(a, b)
 
 
 def test_range_limits_and_special_values(check):
