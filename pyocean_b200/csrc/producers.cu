@@ -372,7 +372,7 @@ __global__ void PPM_BOUNDS ppm_final_kernel(PPMArgs a, double* __restrict__ out)
 
 // One face's whole correction by the general passes' arithmetic, read from memory layer by layer: the faces of
 // ppm_newton_kernel outside the ranges of its short quotients (velocities or widths that are not finite, or whose
-// exponents are beyond +-250).
+// exponents are beyond +-250; corrections below 2^-650).
 static __device__ __noinline__ void ppm_face_general(const PPMArgs& a, int o, int steps, int max_iter, bool mark,
                                                      double* __restrict__ out)
 {
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     double* shU = shD + 32 * ROWS;
     double* shL = shU + 32 * ROWS;
     double* row = shL + 32 * ROWS;                 // te, tw, du / R, den
-    __shared__ int command;                        // 1: evaluate at du; 0: done
+    __shared__ int command;                        // 1: evaluate at du; 0: done; -1: outside the short quotients
     int steps = max_iter;
     if (check) {
         int last = 0;                              // the reference's steps: up to the first that left no face
@@ -536,7 +536,9 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     // the velocities; the bracket over this warp's layers; whether the short quotients serve this CTA
     const double limw = 0.5 * fc.dxw / a.dt, lime = 0.5 * fc.dxe / a.dt;
     double mnw = INFINITY, mxe = -INFINITY;
-    auto mid = [](double x) {                      // |x| in [2^-250, 2^250): no quotient below leaves the range
+    // |x| in [2^-250, 2^250): a Courant number |u + du| dt / dx is then a quotient in range, or zero, unless u = 0 and du
+    // is tiny (checked with each step): a sum of two numbers does not cancel below their last bit
+    auto mid = [](double x) {
         return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (773u << 20) < (500u << 20);
     };
     bool odd = open && !(mid(dxw) && mid(dxe) && mid(a.dt) && dxw > 0.0 && dxe > 0.0 && a.dt > 0.0);
@@ -610,11 +612,13 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
                 du = nw;
                 const bool moved = in && (it < 0 || __double_as_longlong(nw) != __double_as_longlong(d));
                 go = __any_sync(0xffffffffu, moved);
+                const unsigned size = (unsigned)__double2hiint(nw) & 0x7fffffffu;
+                if (__any_sync(0xffffffffu, open && nw != 0.0 && size < (1023u - 650u) << 20)) go = -1;
                 // every later step of these faces repeats the last one
-                if (!go && !check && __any_sync(0xffffffffu, left) && lane == 0)
+                if (go == 0 && !check && __any_sync(0xffffffffu, left) && lane == 0)
                     for (int m = it + 1; m < max_iter; ++m) a.unconverged[m] = 1;
             }
-            if (go) {
+            if (go > 0) {
                 row[2 * 32] = du;
             } else {                               // the residual's share (cnuity.F90 style, ale.py:718-740)
                 const double R = q - s, te = row[0], tw = row[32];
@@ -631,8 +635,12 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
             if (lane == 0) command = go;
         }
         __syncthreads();
-        if (!command) break;
+        if (command <= 0) break;
         evaluate(row[2 * 32], true);
+    }
+    if (command < 0) {
+        if (wp == 0 && in) ppm_face_general(a, o, steps, max_iter, !check, out);
+        return;
     }
     // final fluxes
     if (in) {
