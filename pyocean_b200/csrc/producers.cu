@@ -432,22 +432,36 @@ static __device__ __noinline__ void ppm_face_general(const PPMArgs& a, int o, in
 // through shared memory, and the first warp adds them and their derivatives over the layers in the reference's order
 // and takes the step of its lane's face.  A layer whose velocity changes sign reloads the other side.
 //
-// The reference stops when every face of the grid has converged, which a CTA cannot know: the launch with check = 0
-// runs max_iter steps and marks in `unconverged` each step after which one of its faces had not converged; the launch
-// with check = 1 finds the step the reference stops at and, where that is before max_iter, runs the CTA again up to
-// there.  A face whose correction comes out unchanged stays as it is (its state repeats), so a CTA whose faces are all
-// there leaves its loop.
+// The reference stops at the first step after which every face of the grid has converged, T, which a CTA cannot know.  A
+// face not converged after a step marks it in `unconverged`.  A face whose correction comes out unchanged stays as it is
+// (its state repeats), so a CTA whose faces are all there leaves its loop: it is settled for every later step.
+//
+// Up to 52 layers, two launches (PPM_PLAIN): with check = 0 every CTA runs all steps, or until it is settled, and marks them;
+// with check = 1, where T, the first step left unmarked, is not the last one, every CTA runs again up to it.  For deeper
+// columns two others come first:
+//   PPM_FIRST   as check = 0, but once PPM_SCOUTS CTAs have ended, a CTA stops at the first step that was unmarked when it
+//               began and after which its own faces have converged (unless that is a late one: then some face of the grid
+//               will hardly ever converge), and keeps its corrections and brackets;
+//   PPM_RESUME  the CTAs that are not at T go on to it, or run again up to it; one that finds a face not converged at T (it
+//               had been: rounding) sets unconverged[max_iter], and only then the plain launches follow.
+// A mark always tells the truth, so the result does not depend on the order in which the CTAs run.
 //
 // What bounds it: latency, with registers and shared memory for 16 warps an SM: the sums over the layers, which only
-// other CTAs' work hides (CTAS of them fit an SM), and the loads of sides that changed (issue slots are 31 % busy).  1.24 ms
-// for 20 steps at 512 x 512 x 50; 1.29 with a test of every layer's velocity for its side in each step and 5 layers a
-// batch of the sums' loads.  As one launch per step, each re-reading
-// 0.63 GB, the 22 passes took 3.55 ms (158 us per step).
-template <int LPT, int W, int CTAS>
-__global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int max_iter, int check,
-                                                                  double* __restrict__ out)
+// other CTAs' work hides (CTAS of them fit an SM), and the loads of sides that changed (issue slots are 31 % busy).  20 steps
+// at 512 x 512 x 50 take 1.24 ms; 1.29 with a test of every layer's velocity for its side in each step and 5 layers a
+// batch of the sums' loads.  As one launch per step, each re-reading 0.63 GB, the 22 passes took 3.55 ms (158 us per step).
+// A 512 x 512 transport's launches, for noise (T is the last step) and for columns of one direction (T = 5):
+//   75 layers   all four 2.02 and 2.22 ms, the plain two 1.97 and 3.32;
+//   50 layers   all four 1.37 and 1.11 ms, the plain two 1.29 and 2.05.  Grids of real flows nearly always hold a face whose
+//               transport is too small to converge, so these columns take the two.
+enum PPMPass { PPM_PLAIN, PPM_FIRST, PPM_RESUME };
+constexpr int PPM_SCOUTS = 512;                   // CTAs that have ended before others stop early
+constexpr int PPM_SOON = 8;                       // with more steps marked than these T is expected to be the last one
+
+template <int LPT, int W, int PASS>
+__device__ __forceinline__ void ppm_newton_faces(const PPMArgs& a, int max_iter, int check, int block, double* sh,
+                                                 double* __restrict__ out)
 {
-    extern __shared__ double sh[];
     constexpr int ROWS = LPT * W;                  // rows of 32 lanes: F, dF, u, limit (ROWS each), then
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, n = a.n;
     double* shF = sh + lane;
@@ -456,24 +470,37 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     double* shL = shU + 32 * ROWS;
     double* row = shL + 32 * ROWS;                 // te, tw, du / R, den
     __shared__ int command;                        // 1: evaluate at du; 0: done; -1: outside the short quotients
-    int steps = max_iter;
-    if (check) {
-        int last = 0;                              // the reference's steps: up to the first that left no face
-        for (; last < max_iter; last += 32) {
-            const bool none = last + lane < max_iter && *(volatile int*)(a.unconverged + last + lane) == 0;
+    const bool marks = PASS == PPM_FIRST || (PASS == PPM_PLAIN && !check);
+    // the steps from m on that are marked, up to the first that is not (max_iter: all); by a whole warp
+    auto marked_to = [&](int m) {
+        for (; m < max_iter; m += 32) {
+            const bool none = m + lane < max_iter && *(volatile int*)(a.unconverged + m + lane) == 0;
             const unsigned first = __ballot_sync(0xffffffffu, none);
-            if (first) {
-                last += __ffs(first) - 1;
-                break;
-            }
+            if (first) return m + __ffs(first) - 1;
         }
-        if (last + 1 >= max_iter) return;
-        steps = last + 1;
+        return max_iter;
+    };
+    int stop = max_iter, steps = max_iter, from = -1;      // the unmarked step, the steps to run, the step to go on from
+    if (!marks) {
+        stop = marked_to(0);
+        steps = min(stop + 1, max_iter);
+        if (PASS == PPM_PLAIN && steps == max_iter) return;
     }
     const int nf = a.nx + 1, pf = a.ny * nf;
-    const int o = blockIdx.x * 32 + lane;
+    const int o = block * 32 + lane;
     const bool in = o < pf;
     const int oc = in ? o : pf - 1, j = oc / nf, f = oc - j * nf;
+    if (PASS == PPM_RESUME) {
+        // the block's end in the first pass: step m >= 0; -2: the last one, by the general faces; -3 - f: settled from step f
+        const int end = (int)__ldg(a.err + oc);
+        if (end == steps - 1 || (end == -2 && steps == max_iter) || (end <= -3 && -3 - end <= steps - 1)) return;
+        from = end >= 0 && end < steps - 1 ? end : -1;
+    }
+    int known = 0;                                 // the steps before it are marked
+    if (PASS == PPM_FIRST && wp == 0) {
+        known = *(volatile int*)(a.unconverged + max_iter) < PPM_SCOUTS ? max_iter : marked_to(0);
+        if (known > PPM_SOON) known = max_iter;
+    }
     const FaceCells fc = face_cells(a, j, f);
     const bool open = in && fc.aw && fc.ae;
     const int k0 = wp * LPT;
@@ -554,20 +581,24 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
         shL[(k0 + l) * 32] = INFINITY;
     }
     if (__syncthreads_or(odd)) {
-        if (wp == 0 && in) ppm_face_general(a, o, steps, max_iter, !check, out);
+        if (wp == 0 && in) {
+            ppm_face_general(a, o, steps, max_iter, marks, out);
+            if (PASS == PPM_FIRST) a.err[o] = -2.0;
+        }
         return;
     }
+    const double du0 = from >= 0 ? __ldg(a.du + oc) : 0.0;
     if (open) {
 #pragma unroll
         for (int l = 0; l < LPT; ++l)
-            if (k0 + l < n) load_side(l, shU[(k0 + l) * 32] >= 0.0);
+            if (k0 + l < n) load_side(l, (from >= 0 ? shU[(k0 + l) * 32] + du0 : shU[(k0 + l) * 32]) >= 0.0);
     } else {
         west = ~0u;
     }
     shF[wp * 32] = mnw;
     shD[wp * 32] = mxe;
     __syncthreads();
-    double hi, lo, du = 0.0, err = 0.0, ds = 0.0, s = 0.0, q = 0.0;       // the first warp's: its lanes' faces
+    double hi, lo, du = du0, err = 0.0, ds = 0.0, s = 0.0, q = 0.0;       // the first warp's: its lanes' faces
     if (wp == 0) {
         mnw = INFINITY;
         mxe = -INFINITY;
@@ -577,6 +608,10 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
         }
         hi = pmax(pmin(limw, mnw), 0.0);
         lo = pmin(pmax(-lime, mxe), 0.0);
+        if (from >= 0) {
+            hi = __ldg(a.hi + oc);
+            lo = __ldg(a.lo + oc);
+        }
         q = in ? __ldg(a.Q_bt + oc) : 0.0;
     } else if (wp >= W - 2) {                      // the face's transport thicknesses, for the residual's share
         const double* qs = wp == W - 2 ? a.q_e : a.q_w;
@@ -585,8 +620,8 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
         row[(wp == W - 2 ? 0 : 1) * 32] = acc;
     }
     __syncthreads();
-    evaluate(0.0, steps == 0);
-    for (int it = -1;; ++it) {                     // it: the step just evaluated (-1: the given velocities)
+    evaluate(du0, from >= 0 || steps == 0);
+    for (int it = from;; ++it) {                   // it: the step just evaluated (-1: the given velocities)
         __syncthreads();
         if (wp == 0) {
             double s2 = 0.0, d2 = 0.0;
@@ -599,9 +634,10 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
             err = s2 - q;
             ds = d2;
             const bool left = in && fabs(err) > 1e-12 * pmax(fabs(q), 1.0);
-            if (it >= 0 && !check && __any_sync(0xffffffffu, left) && lane == 0) a.unconverged[it] = 1;
-            int go = 0;
-            if (it + 1 < steps) {
+            if (marks && it > from && __any_sync(0xffffffffu, left) && lane == 0) a.unconverged[it] = 1;
+            if (PASS == PPM_RESUME && it == stop && __any_sync(0xffffffffu, left) && lane == 0) a.unconverged[max_iter] = -1;
+            int go = 0, at = it;
+            if (it + 1 < steps && !(PASS == PPM_FIRST && it >= known && !__any_sync(0xffffffffu, left))) {
                 const double d = du;
                 if (err > 0.0) hi = d;
                 if (err < 0.0) lo = d;
@@ -615,8 +651,17 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
                 const unsigned size = (unsigned)__double2hiint(nw) & 0x7fffffffu;
                 if (__any_sync(0xffffffffu, open && nw != 0.0 && size < (1023u - 650u) << 20)) go = -1;
                 // every later step of these faces repeats the last one
-                if (go == 0 && !check && __any_sync(0xffffffffu, left) && lane == 0)
+                if (go == 0) at = -3 - it;
+                if (go == 0 && marks && __any_sync(0xffffffffu, left) && lane == 0)
                     for (int m = it + 1; m < max_iter; ++m) a.unconverged[m] = 1;
+                if (PASS == PPM_RESUME && go == 0 && stop < max_iter && __any_sync(0xffffffffu, left) && lane == 0)
+                    a.unconverged[max_iter] = -1;
+            }
+            if (go <= 0 && PASS == PPM_FIRST && in) {
+                a.du[o] = du;
+                a.hi[o] = hi;
+                a.lo[o] = lo;
+                a.err[o] = go < 0 ? -2.0 : (double)at;
             }
             if (go > 0) {
                 row[2 * 32] = du;
@@ -639,7 +684,7 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
         evaluate(row[2 * 32], true);
     }
     if (command < 0) {
-        if (wp == 0 && in) ppm_face_general(a, o, steps, max_iter, !check, out);
+        if (wp == 0 && in) ppm_face_general(a, o, steps, max_iter, marks, out);
         return;
     }
     // final fluxes
@@ -652,17 +697,53 @@ __global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int
     }
 }
 
-template <int LPT, int W, int CTAS>
-static cudaError_t ppm_newton_launch(const PPMArgs& a, int max_iter, double* out, cudaStream_t st)
+// EARLY: the launches of deep columns.  Their blocks of faces are taken in 64 strides, so that the first CTAs see the whole
+// grid; the plain launches, which hardly ever have work then, take few CTAs that go through the blocks.
+template <int LPT, int W, int CTAS, int PASS, bool EARLY>
+__global__ void __launch_bounds__(32 * W, CTAS) ppm_newton_kernel(PPMArgs a, int max_iter, int check, int blocks,
+                                                                  double* __restrict__ out)
 {
-    const unsigned g = (unsigned)(((i64)a.ny * (a.nx + 1) + 31) / 32);
+    extern __shared__ double sh[];
+    if (!EARLY) {
+        ppm_newton_faces<LPT, W, PASS>(a, max_iter, check, blockIdx.x, sh, out);
+    } else if (PASS != PPM_PLAIN) {
+        const int b = blockIdx.x % 64 * (gridDim.x / 64) + blockIdx.x / 64;
+        if (b < blocks) ppm_newton_faces<LPT, W, PASS>(a, max_iter, check, b, sh, out);
+        if (PASS == PPM_FIRST && threadIdx.x == 0 && blockIdx.x < PPM_SCOUTS) atomicAdd(a.unconverged + max_iter, 1);
+    } else if (*(volatile int*)(a.unconverged + max_iter) == -1) {
+        for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
+            ppm_newton_faces<LPT, W, PASS>(a, max_iter, check, b, sh, out);
+            __syncthreads();
+        }
+    }
+}
+
+template <int LPT, int W, int CTAS, int PASS, bool EARLY>
+static cudaError_t ppm_newton_pass(const PPMArgs& a, int max_iter, int check, double* out, cudaStream_t st)
+{
+    const int blocks = (int)(((i64)a.ny * (a.nx + 1) + 31) / 32), few = 148 * CTAS;
     constexpr size_t shmem = (size_t)(4 * LPT * W + 4) * 32 * sizeof(double);
-    const auto kernel = ppm_newton_kernel<LPT, W, CTAS>;
+    const auto kernel = ppm_newton_kernel<LPT, W, CTAS, PASS, EARLY>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
     if (e != cudaSuccess) return e;
-    kernel<<<g, 32 * W, shmem, st>>>(a, max_iter, 0, out);
-    if (max_iter > 1) kernel<<<g, 32 * W, shmem, st>>>(a, max_iter, 1, out);
+    const int grid = !EARLY ? blocks : (PASS == PPM_PLAIN ? (blocks < few ? blocks : few) : (blocks + 63) / 64 * 64);
+    kernel<<<grid, 32 * W, shmem, st>>>(a, max_iter, check, blocks, out);
     return cudaSuccess;
+}
+
+template <int LPT, int W, int CTAS, bool EARLY>
+static cudaError_t ppm_newton_launch(const PPMArgs& a, int max_iter, double* out, cudaStream_t st)
+{
+    if (EARLY) {
+        cudaError_t e = ppm_newton_pass<LPT, W, CTAS, EARLY ? PPM_FIRST : PPM_PLAIN, EARLY>(a, max_iter, 0, out, st);
+        if (max_iter <= 1) return e;
+        if (e == cudaSuccess)
+            e = ppm_newton_pass<LPT, W, CTAS, EARLY ? PPM_RESUME : PPM_PLAIN, EARLY>(a, max_iter, 0, out, st);
+        if (e != cudaSuccess) return e;
+    }
+    const cudaError_t e = ppm_newton_pass<LPT, W, CTAS, PPM_PLAIN, EARLY>(a, max_iter, 0, out, st);
+    if (e != cudaSuccess || max_iter <= 1) return e;
+    return ppm_newton_pass<LPT, W, CTAS, PPM_PLAIN, EARLY>(a, max_iter, 1, out, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1182,10 +1263,12 @@ extern "C" int pocean_ppm_transport_f64(const double* h, const double* ut, const
     if (nz <= 80) {
         // layers per warp, warps, CTAs per SM: four warps and as many CTAs as registers and shared memory hold are the
         // fastest split (whole layer-transport step at 512 x 512 x 50: 3.87 ms; 7 layers x 8 warps x 3 CTAs 4.44,
-        // 5 x 12 x 2 4.24, 10 x 5 x 3 3.98): what a CTA's sums leave idle, the other CTAs fill
-        e = nz <= 32 ? pr::ppm_newton_launch<8, 4, 5>(a, max_iter, Qx, st)
-                     : (nz <= 52 ? pr::ppm_newton_launch<13, 4, 4>(a, max_iter, Qx, st)
-                                 : pr::ppm_newton_launch<20, 4, 2>(a, max_iter, Qx, st));
+        // 5 x 12 x 2 4.24, 10 x 5 x 3 3.98): what a CTA's sums leave idle, the other CTAs fill.  Above 52 layers two CTAs
+        // are left, and twice the warps load a face's layers faster: 512 x 512 x 75, all steps of noise: 10 layers x 8 warps
+        // 1.92 ms, 20 x 4 3.08, 16 x 5 3.38, 8 x 10 2.03.
+        e = nz <= 32 ? pr::ppm_newton_launch<8, 4, 5, false>(a, max_iter, Qx, st)
+                     : (nz <= 52 ? pr::ppm_newton_launch<13, 4, 4, false>(a, max_iter, Qx, st)
+                                 : pr::ppm_newton_launch<10, 8, 2, true>(a, max_iter, Qx, st));
         if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
         return pocean_check_launch(fn);
     }
