@@ -160,8 +160,9 @@ static __device__ __noinline__ void general_column(const double* h, const double
     rc::remap_column_general<NMAX>(io, 0, n0, n1, scheme);
 }
 
-// Columns c0 .. c0 + SG_COLS - 1 of fields m0 .. m0 + NF - 1.
-template <int NF>
+// Columns c0 .. c0 + SG_COLS - 1 of fields m0 .. m0 + NF - 1.  MARK: columns with a negative or NaN target thickness are left
+// to a launch of their own, as by the sweep.
+template <int NF, bool MARK>
 __device__ __forceinline__ void remap_segments_body(double* sm, const double* __restrict__ h_src,
                                                     const double* __restrict__ f_src, const double* __restrict__ h_tgt,
                                                     const uint8_t* __restrict__ wet_in, int n0, int n1, i64 plane,
@@ -283,17 +284,19 @@ __device__ __forceinline__ void remap_segments_body(double* sm, const double* __
     __syncthreads();
     const int na = s_active[x], fst = s_first[x], lst = s_last[x];
     const bool run = wet && s_regular[x] && na > 0;
-    if (wet && !run) {
+    if (wet && !s_regular[x]) {                                // a negative or NaN target thickness
+        if (slot < NF) {
+            const double* fm = f + (i64)slot * n0 * plane;
+            double* om = o + (i64)slot * n1 * plane;
+            if (MARK) om[0] = __longlong_as_double(kRedo);
+            else if (mx <= 64) general_column<64>(hs, fm, ht, om, plane, n0, n1, scheme);
+            else general_column<SG_LAYERS>(hs, fm, ht, om, plane, n0, n1, scheme);
+        }
+    } else if (wet && !run) {                                  // no active cell (remap.py:375-381)
 #pragma unroll
         for (int m = 0; m < NF; ++m) {
-            const double* fm = f + (i64)m * n0 * plane;
             double* om = o + (i64)m * n1 * plane;
-            if (!s_regular[x]) {                               // a negative or NaN target thickness
-                if (slot == 0) {
-                    if (mx <= 64) general_column<64>(hs, fm, ht, om, plane, n0, n1, scheme);
-                    else general_column<SG_LAYERS>(hs, fm, ht, om, plane, n0, n1, scheme);
-                }
-            } else if (n0 == n1) {                             // no active cell (remap.py:375-381)
+            if (n0 == n1) {
                 for (int k = slot; k < n1; k += SG_SLOTS) om[k * plane] = at(m, fu + k);
             } else {
                 double mean = 0.0;
@@ -467,19 +470,20 @@ __device__ __forceinline__ void remap_segments_body(double* sm, const double* __
 // CTAS (resident CTAs per SM, which sets the registers): 4; for one field of a column, whose shared memory leaves room for
 // more up to about 60 layers, 5 (512 x 512 x 50: 653 us against 675 at 4; 320 x 320 x 75: 398 at 4, 440 at 5).
 constexpr size_t SG_FIVE = 44 * 1024;
-template <int NF, int CTAS>
+template <int NF, int CTAS, bool MARK>
 __global__ void __launch_bounds__(SG_THREADS, CTAS) remap_segments_kernel(
     const double* __restrict__ h_src, const double* __restrict__ f_src, const double* __restrict__ h_tgt,
     const uint8_t* __restrict__ wet, int n0, int n1, i64 plane, int field0, int scheme, double* __restrict__ out)
 {
     extern __shared__ double sm[];
-    remap_segments_body<NF>(sm, h_src, f_src, h_tgt, wet, n0, n1, plane, field0 + (int)blockIdx.y * NF, scheme, out,
-                            (i64)blockIdx.x * SG_COLS);
+    remap_segments_body<NF, MARK>(sm, h_src, f_src, h_tgt, wet, n0, n1, plane, field0 + (int)blockIdx.y * NF, scheme, out,
+                                  (i64)blockIdx.x * SG_COLS);
 }
 
 // The same over every field of every domain of a batch (its advected stack, D.a.out -> D.rout).  A CTA goes through
 // SG_BATCH_COLS columns of one domain, which its first thread finds.
 constexpr int SG_BATCH_COLS = 32;
+template <bool MARK>
 __global__ void __launch_bounds__(SG_THREADS, 4) remap_segments_batched(const BatchDomain* __restrict__ doms,
                                                                        const int* __restrict__ off, int ndom)
 {
@@ -494,7 +498,7 @@ __global__ void __launch_bounds__(SG_THREADS, 4) remap_segments_batched(const Ba
     const int m = local / groups;
     i64 c = (i64)(local - m * groups) * SG_BATCH_COLS;
     for (const i64 end = c + SG_BATCH_COLS; c < end && c < plane; c += SG_COLS) {
-        remap_segments_body<1>(sm, D.h_src, D.a.out, D.h_tgt, D.wet, n, n, plane, m, D.remap_scheme, D.rout, c);
+        remap_segments_body<1, MARK>(sm, D.h_src, D.a.out, D.h_tgt, D.wet, n, n, plane, m, D.remap_scheme, D.rout, c);
         __syncthreads();
     }
 }
@@ -527,10 +531,10 @@ __global__ void __launch_bounds__(128) remap_general_batched(const BatchDomain* 
     const BatchDomain& D = doms[d];
     const Shape s = D.a.s;
     const i64 plane = (i64)s.ny * s.nx;
-    const int cblocks = (int)((plane + 127) / 128);
+    const int cblocks = (int)((plane + blockDim.x - 1) / blockDim.x);      // the columns of a CTA of `off`
     const int local = blockIdx.x - __ldg(off + d);
     const int m = local / cblocks;
-    const i64 c = (i64)(local - m * cblocks) * 128 + threadIdx.x;
+    const i64 c = (i64)(local - m * cblocks) * blockDim.x + threadIdx.x;
     if (c >= plane) return;
     remap_general_body<NMAX>(D.h_src, D.a.out, D.h_tgt, s.n, s.n, plane, m, D.remap_scheme, D.rout, c);
 }
@@ -566,6 +570,13 @@ __global__ void __launch_bounds__(128) reconstruct_kernel(const double* __restri
 // two steps 1.71 ms by the sweep, 1.47 ms side by side).
 bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::SG_LAYERS && columns <= 150000; }
 
+// Whether the columns with a negative or NaN target thickness of `columns` (those of all fields) of up to n layers take a
+// launch of their own.  Else a thread of their CTA does them while the others wait.  The launch costs 3 us, at this line 4 %
+// of the remap; without it, 360 x 360 x 50 columns of two fields, one in a hundred of them such, take 2.24 ms instead of
+// 0.96, all of them 15.1 instead of 1.5 (by the sweep 1.30 and 1.40), and 64 x 64 x 50 of one field 0.31 and 0.28 ms (by the
+// sweep 0.49 and 0.29).
+static bool irregular_launch(long long columns, int n) { return columns * n > 1000000; }
+
 // Columns of a batched remap CTA.
 int remap_batched_columns(bool segments) { return segments ? remap::SG_BATCH_COLS : 128; }
 
@@ -589,9 +600,14 @@ cudaError_t remap_batched_launch(const BatchDomain* doms, const int* off_dev, co
     auto offs = [&](int pass) { return off_dev + pass * (ndom + 1); };
     if (segments) {
         const size_t smem = remap::segment_smem(1, nmax, nmax);
-        const cudaError_t e = allow_smem((const void*)remap::remap_segments_batched, SG_SMEM1);
+        const bool mark = irregular_launch((long long)total(BP_RALL) * remap::SG_BATCH_COLS, nmax);
+        const auto kernel = mark ? remap::remap_segments_batched<true> : remap::remap_segments_batched<false>;
+        const cudaError_t e = allow_smem((const void*)kernel, SG_SMEM1);
         if (e != cudaSuccess) return e;
-        remap::remap_segments_batched<<<total(BP_RALL), remap::SG_THREADS, smem, st>>>(doms, offs(BP_RALL), ndom);
+        kernel<<<total(BP_RALL), remap::SG_THREADS, smem, st>>>(doms, offs(BP_RALL), ndom);
+        if (mark)
+            remap::remap_general_batched<remap::SG_LAYERS>
+                <<<total(BP_RALL), remap::SG_BATCH_COLS, 0, st>>>(doms, offs(BP_RALL), ndom);
         return cudaSuccess;
     }
     if (nf_mode == 2) {
@@ -648,8 +664,11 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
         const int threads = remap::segment_threads(n0, n1);
         const dim3 g((unsigned)((plane + remap::SG_COLS - 1) / remap::SG_COLS), (unsigned)nf2);
         const size_t s1 = remap::segment_smem(1, n0, n1), s2 = remap::segment_smem(2, n0, n1);
-        const auto one = s1 <= remap::SG_FIVE ? remap::remap_segments_kernel<1, 5> : remap::remap_segments_kernel<1, 4>;
-        const auto two = remap::remap_segments_kernel<2, 4>;
+        const bool mark = irregular_launch((long long)plane * nfields, n0 > n1 ? n0 : n1), five = s1 <= remap::SG_FIVE;
+        const auto one = mark ? (five ? remap::remap_segments_kernel<1, 5, true> : remap::remap_segments_kernel<1, 4, true>)
+                              : (five ? remap::remap_segments_kernel<1, 5, false>
+                                      : remap::remap_segments_kernel<1, 4, false>);
+        const auto two = mark ? remap::remap_segments_kernel<2, 4, true> : remap::remap_segments_kernel<2, 4, false>;
         cudaError_t e = rest ? allow_smem((const void*)one, SG_SMEM1) : cudaSuccess;
         if (e == cudaSuccess && nf2) e = allow_smem((const void*)two, SG_SMEM2);
         if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
@@ -657,6 +676,7 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
         if (rest)
             one<<<dim3(g.x, (unsigned)rest), threads, s1, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 2 * nf2, scheme,
                                                                 out);
+        if (mark) remap_general_launch(h_src, f_src, h_tgt, n0, n1, plane, nfields, scheme, out, st);
         return pocean_check_launch(fn);
     }
     const unsigned gx = (unsigned)((plane + 127) / 128);

@@ -20,14 +20,14 @@ FCT_LAUNCHES = 8
 
 def remap_launches(nt: int, n: int, n1: int, columns: int) -> int:
     """Kernel launches of a remap of nt fields of ``columns`` columns from n to n1 layers: the field pairs and the single
-    fields and, by the sweep, the general-column fixup.  The rule is ``pocean_remap_columns_f64``'s in csrc/remap.cu."""
+    fields and, by the sweep or of many columns, the general-column fixup.  The rule is ``pocean_remap_columns_f64``'s in csrc/remap.cu."""
     deep = max(n, n1)
     pair_bytes = 8 * ((3 * n + n1 + 2 + 2 * (4 * n + 1 + 2 * deep)) * 8 + 2 * n + n1 + 8)
     fit2 = pair_bytes <= 72 * 1024
     if deep > 96 or not (fit2 or nt == 1 or columns < 150000):
         return (nt >= 2) + (nt % 2) + 1
     pairs = nt // 2 if fit2 else 0
-    return (pairs > 0) + (nt > 2 * pairs)
+    return (pairs > 0) + (nt > 2 * pairs) + (columns * nt * deep > 1000000)
 
 
 class ALETracerStep:
