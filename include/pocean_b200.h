@@ -184,6 +184,9 @@ int pocean_advect_rhs_f64(const double* c, const double* Qx, const double* Qy, c
 int pocean_remap_columns_f64(const double* h_src, const double* f_src, const double* h_tgt, const uint8_t* wet,
                              int n0, int n1, int ny, int nx, int nfields, int scheme, double* out, void* stream);
 
+/* Kernel launches of a pocean_remap_columns_f64 call of these sizes. */
+int pocean_remap_launches(int n0, int n1, int ny, int nx, int nfields);
+
 /*
  * reconstruct (core/vertical/remap.py:234-294) of ncols columns of n cells: h and u (n, ncols), coef (n, ncols, 3),
  * the coefficients (c0, c1, c2) of p(xi) = c0 + c1 xi + c2 xi^2 in each cell with the reference's default
@@ -413,6 +416,9 @@ int pocean_batch_create(const pocean_domain* domains, int ndom, int tile_rows, v
 /* Enqueues one step of every domain.  remap_nf: fields per remap thread (1 or 2, a tuning parameter); mixed: FP32
  * WENO weights (pocean_advect_fct_mixed) instead of FP64. */
 int pocean_batch_step(const pocean_batch* b, int parity, int remap_nf, int mixed, void* stream);
+
+/* Kernel launches of a pocean_batch_step over ndom domains of these shapes: (nt, nz, ny, nx) of each in turn. */
+int pocean_batch_launches(const int* shapes, int ndom, int remap_nf);
 
 void pocean_batch_destroy(pocean_batch* b);
 

@@ -79,6 +79,8 @@ SIGNATURES: dict[str, tuple] = {
     "pocean_batch_device_bytes": (_Z, [_I]),
     "pocean_batch_create": (_I, [_P, _I, _I, _P, _Z, ctypes.POINTER(_P), _P]),
     "pocean_batch_step": (_I, [_P, _I, _I, _I, _P]),
+    "pocean_batch_launches": (_I, [_P, _I, _I]),
+    "pocean_remap_launches": (_I, [_I, _I, _I, _I, _I]),
     "pocean_batch_destroy": (None, [_P]),
 }
 

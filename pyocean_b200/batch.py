@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .step import FCT_LAUNCHES, remap_launches
+from .step import FCT_LAUNCHES
 
 
 class _Domain(ctypes.Structure):
@@ -221,27 +221,15 @@ class DomainBatch:
 
 
 def batch_launches(shapes: Sequence[tuple], remap_nf: int) -> int:
-    """Kernel launches of one batched step of domains of these (nt, n, ny, nx) shapes: the FCT passes, one launch each
-    per 64 domains (large batches of one tracer limit in one pass instead of two, ``limit_in_one_pass`` in
-    csrc/advect.cu), then the remap: of a batch that leaves the chip room (``remap_batch_segments`` in csrc/remap.cu) one
-    launch over every field (and the general-column fixup where there are many columns), else one over field pairs and one over the odd fields (or one over all fields) and the
-    general-column fixup."""
-    fct = 0
-    for g in range(0, len(shapes), 64):
-        group = shapes[g:g + 64]
-        one_pass = all(s[0] == 1 for s in group) and sum(s[1] * s[2] * s[3] for s in group) >= 1 << 21
-        fct += FCT_LAUNCHES - one_pass
-    nmax = max(s[1] for s in shapes)
-    if nmax <= 96 and sum(s[0] * s[2] * s[3] for s in shapes) <= 150000:
-        return fct + 1 + (sum(-(-s[2] * s[3] // 32) * 32 * s[0] for s in shapes) * nmax > 1000000)
-    if remap_nf == 2:
-        return fct + any(s[0] >= 2 for s in shapes) + any(s[0] % 2 for s in shapes) + 1
-    return fct + 2
+    """Kernel launches of one batched step of domains of these (nt, n, ny, nx) shapes."""
+    flat = [int(x) for s in shapes for x in s]
+    return _lib.lib().pocean_batch_launches((ctypes.c_int * len(flat))(*flat), len(shapes), remap_nf)
 
 
 def sequential_launches(domains: Sequence[Domain]) -> int:
     """Kernel launches of one ``sequential_step``: per domain the FCT passes and the remap's launches."""
-    return sum(FCT_LAUNCHES + remap_launches(d.shape[0], d.shape[1], d.shape[1], d.shape[2] * d.shape[3]) for d in domains)
+    L = _lib.lib()
+    return sum(FCT_LAUNCHES + L.pocean_remap_launches(n, n, ny, nx, nt) for nt, n, ny, nx in (d.shape for d in domains))
 
 
 def sequential_step(domains: Sequence[Domain], parity: int, mixed: bool = False, stream: int | None = None) -> None:

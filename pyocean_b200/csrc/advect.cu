@@ -1162,14 +1162,35 @@ static void fct_batched_stages(FctBatch& B, cudaStream_t st)
 // Whether one marching pass limits a launch's domains instead of the coefficient and the final pass: with one tracer
 // each and enough cells that its long warps fill the chip.  Batches of 0.7 M cells 416 us a step with the two passes, 428
 // with one; 2.6 M 1373 and 1366; 7.9 M 3740 and 3700; 18.9 M 7726 and 7559.
+static bool limit_in_one_pass(bool one_tracer, i64 cells) { return one_tracer && cells >= (1ll << 21); }
+
 static bool limit_in_one_pass(const FctBatch& B)
 {
+    bool one = true;
     i64 cells = 0;
     for (int d = 0; d < B.ndom; ++d) {
-        if (B.a[d].s.nt > 1) return false;
+        one = one && B.a[d].s.nt == 1;
         cells += (i64)B.a[d].s.n * B.a[d].s.ny * B.a[d].s.nx;
     }
-    return cells >= (1ll << 21);
+    return limit_in_one_pass(one, cells);
+}
+
+// Kernel launches of fct_batched_launch for domains of these shapes (nt, nz, ny, nx): classes, two face and cell passes, the
+// third face pass and the limiter's one or two, per BATCH_CAP domains.
+int fct_batch_launches(const int* shapes, int ndom)
+{
+    int total = 0;
+    for (int d0 = 0; d0 < ndom; d0 += BATCH_CAP) {
+        bool one = true;
+        i64 cells = 0;
+        for (int d = d0; d < ndom && d < d0 + BATCH_CAP; ++d) {
+            const int* s = shapes + 4 * d;
+            one = one && s[0] == 1;
+            cells += (i64)s[1] * s[2] * s[3];
+        }
+        total += limit_in_one_pass(one, cells) ? 7 : 8;
+    }
+    return total;
 }
 
 template <bool ZV, bool MIX>

@@ -130,6 +130,12 @@ extern "C" int pocean_batch_create(const pocean_domain* domains, int ndom, int t
     return POCEAN_OK;
 }
 
+extern "C" int pocean_batch_launches(const int* shapes, int ndom, int remap_nf)
+{
+    if (!shapes || ndom < 1) return 0;
+    return fct_batch_launches(shapes, ndom) + remap_batch_launches(shapes, ndom, remap_nf);
+}
+
 extern "C" int pocean_batch_step(const pocean_batch* b, int parity, int remap_nf, int mixed, void* stream)
 {
     const char* fn = "pocean_batch_step";

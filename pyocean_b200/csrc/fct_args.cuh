@@ -103,6 +103,8 @@ void carve_fct_workspace(StepArgs& a, void* workspace);
 // the remap) on the device.
 cudaError_t fct_batched_launch(const BatchDomain* doms_host, int ndom, bool zv, bool mixed, int tile_rows,
                                cudaStream_t st);
+int fct_batch_launches(const int* shapes, int ndom);
+int remap_batch_launches(const int* shapes, int ndom, int nf_mode);
 bool remap_batch_segments(long long columns, int nmax);
 int remap_batched_columns(bool segments);
 cudaError_t remap_batched_launch(const BatchDomain* doms, const int* off_dev, const int* off_host, int ndom, int nf_mode,

@@ -570,6 +570,10 @@ __global__ void __launch_bounds__(128) reconstruct_kernel(const double* __restri
 // two steps 1.71 ms by the sweep, 1.47 ms side by side).
 bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::SG_LAYERS && columns <= 150000; }
 
+// The most dynamic shared memory a side-by-side launch takes: columns of SG_LAYERS layers of one field; field pairs up to
+// three CTAs an SM.
+constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_LAYERS), SG_SMEM2 = 72 * 1024;
+
 // Whether the columns with a negative or NaN target thickness of `columns` (those of all fields) of up to n layers take a
 // launch of their own.  Else a thread of their CTA does them while the others wait.  The launch costs 3 us, at this line 4 %
 // of the remap; without it, 360 x 360 x 50 columns of two fields, one in a hundred of them such, take 2.24 ms instead of
@@ -577,12 +581,27 @@ bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::S
 // sweep 0.49 and 0.29).
 static bool irregular_launch(long long columns, int n) { return columns * n > 1000000; }
 
+// The launches of a remap: of field pairs and of single fields, side by side or by the sweep, and the irregular columns'.
+struct RemapForm {
+    int pairs, singles;
+    bool side, general;
+    int launches() const { return (pairs > 0) + (singles > 0) + general; }
+};
+
+// Side by side, two fields of a column share the work on its thicknesses while three CTAs fit an SM.  Where they do not
+// (above 70 layers) and the columns fill the chip, the sweep's field pairs are faster: two fields of 512 x 512 x 75
+// take 0.79 ms as two single fields side by side, 0.62 by the sweep; 60 x 60 x 75 with four 24 us against 176.
+static RemapForm remap_form(int n0, int n1, i64 plane, int nfields)
+{
+    const int mx = n0 > n1 ? n0 : n1;
+    const bool fit2 = remap::segment_smem(2, n0, n1) <= SG_SMEM2;
+    if (mx > remap::SG_LAYERS || !(fit2 || nfields == 1 || plane < 150000)) return {nfields / 2, nfields % 2, false, true};
+    const int pairs = fit2 ? nfields / 2 : 0;
+    return {pairs, nfields - 2 * pairs, true, irregular_launch((long long)plane * nfields, mx)};
+}
+
 // Columns of a batched remap CTA.
 int remap_batched_columns(bool segments) { return segments ? remap::SG_BATCH_COLS : 128; }
-
-// The most dynamic shared memory a side-by-side launch takes: columns of SG_LAYERS layers of one field; field pairs up to
-// three CTAs an SM.
-constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_LAYERS), SG_SMEM2 = 72 * 1024;
 
 // A kernel's static and dynamic shared memory together above the default limit (48 KB) has to be asked for.  The limit
 // belongs to the kernel, not to the launch: every call asks for the same, so that no other thread's call lowers it between
@@ -590,6 +609,25 @@ constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_L
 static cudaError_t allow_smem(const void* kernel, size_t most)
 {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
+// Kernel launches of remap_batched_launch for domains of these shapes (nt, nz, ny, nx).
+int remap_batch_launches(const int* shapes, int ndom, int nf_mode)
+{
+    long long columns = 0, padded = 0;
+    int nmax = 1;
+    bool pairs = false, odd = false;
+    for (int d = 0; d < ndom; ++d) {
+        const int nt = shapes[4 * d];
+        const long long plane = (long long)shapes[4 * d + 2] * shapes[4 * d + 3];
+        columns += plane * nt;
+        padded += (plane + remap::SG_BATCH_COLS - 1) / remap::SG_BATCH_COLS * remap::SG_BATCH_COLS * nt;
+        nmax = shapes[4 * d + 1] > nmax ? shapes[4 * d + 1] : nmax;
+        pairs = pairs || nt >= 2;
+        odd = odd || nt % 2 == 1;
+    }
+    if (remap_batch_segments(columns, nmax)) return 1 + irregular_launch(padded, nmax);
+    return (nf_mode == 2 ? (int)pairs + (int)odd : 1) + 1;
 }
 
 // nf_mode 2: field pairs (+ the odd field); nf_mode 1: every field on its own.  nmax: the batch's deepest column.
@@ -655,16 +693,13 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const i64 plane = (i64)ny * nx;
-    // Side by side, two fields of a column share the work on its thicknesses while three CTAs fit an SM.  Where they do not
-    // (above 70 layers) and the columns fill the chip, the sweep's field pairs are faster: two fields of 512 x 512 x 75
-    // take 0.79 ms as two single fields side by side, 0.62 by the sweep; 60 x 60 x 75 with four 24 us against 176.
-    const bool fit2 = remap::segment_smem(2, n0, n1) <= SG_SMEM2;
-    if ((n0 > n1 ? n0 : n1) <= remap::SG_LAYERS && (fit2 || nfields == 1 || plane < 150000)) {
-        const int nf2 = fit2 ? nfields / 2 : 0, rest = nfields - 2 * nf2;
+    const RemapForm form = remap_form(n0, n1, plane, nfields);
+    if (form.side) {
+        const int nf2 = form.pairs, rest = form.singles;
         const int threads = remap::segment_threads(n0, n1);
         const dim3 g((unsigned)((plane + remap::SG_COLS - 1) / remap::SG_COLS), (unsigned)nf2);
         const size_t s1 = remap::segment_smem(1, n0, n1), s2 = remap::segment_smem(2, n0, n1);
-        const bool mark = irregular_launch((long long)plane * nfields, n0 > n1 ? n0 : n1), five = s1 <= remap::SG_FIVE;
+        const bool mark = form.general, five = s1 <= remap::SG_FIVE;
         const auto one = mark ? (five ? remap::remap_segments_kernel<1, 5, true> : remap::remap_segments_kernel<1, 4, true>)
                               : (five ? remap::remap_segments_kernel<1, 5, false>
                                       : remap::remap_segments_kernel<1, 4, false>);
@@ -680,7 +715,7 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
         return pocean_check_launch(fn);
     }
     const unsigned gx = (unsigned)((plane + 127) / 128);
-    const int pairs = nfields / 2;
+    const int pairs = form.pairs;
     // 32-bit offsets within a field when every field (n0 or n1 layers of the plane) holds fewer than 2^31 entries
     const bool small = (i64)(n0 > n1 ? n0 : n1) * plane < (1ll << 31);
     if (pairs > 0) {
@@ -691,7 +726,7 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
             remap::remap_stream_kernel<2, i64><<<dim3(gx, pairs), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1,
                                                                                 plane, 0, scheme, out);
     }
-    if (nfields & 1) {
+    if (form.singles) {
         if (small)
             remap::remap_stream_kernel<1, int><<<dim3(gx, 1), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane,
                                                                             nfields - 1, scheme, out);
@@ -701,6 +736,12 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
     }
     remap_general_launch(h_src, f_src, h_tgt, n0, n1, plane, nfields, scheme, out, st);
     return pocean_check_launch(fn);
+}
+
+extern "C" int pocean_remap_launches(int n0, int n1, int ny, int nx, int nfields)
+{
+    if (n0 < 1 || n1 < 1 || ny < 1 || nx < 1 || nfields < 1) return 0;
+    return remap_form(n0, n1, (i64)ny * nx, nfields).launches();
 }
 
 extern "C" int pocean_reconstruct_f64(const double* h, const double* u, int n, long long ncols, int scheme,

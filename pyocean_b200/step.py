@@ -18,18 +18,6 @@ from . import _lib
 FCT_LAUNCHES = 8
 
 
-def remap_launches(nt: int, n: int, n1: int, columns: int) -> int:
-    """Kernel launches of a remap of nt fields of ``columns`` columns from n to n1 layers: the field pairs and the single
-    fields and, by the sweep or of many columns, the general-column fixup.  The rule is ``pocean_remap_columns_f64``'s in csrc/remap.cu."""
-    deep = max(n, n1)
-    pair_bytes = 8 * ((3 * n + n1 + 2 + 2 * (4 * n + 1 + 2 * deep)) * 8 + 2 * n + n1 + 8)
-    fit2 = pair_bytes <= 72 * 1024
-    if deep > 96 or not (fit2 or nt == 1 or columns < 150000):
-        return (nt >= 2) + (nt % 2) + 1
-    pairs = nt // 2 if fit2 else 0
-    return (pairs > 0) + (nt > 2 * pairs) + (columns * nt * deep > 1000000)
-
-
 class ALETracerStep:
     """advect_fct + PPM_H4 (or PCM / PLM) remap of a (nt, N, ny, nx) stack with preallocated buffers."""
 
@@ -44,7 +32,7 @@ class ALETracerStep:
         self.ws_bytes = L.pocean_advect_fct_workspace_bytes(nt, n, ny, nx)
         self.ws = torch.empty(self.ws_bytes, dtype=torch.uint8, device=self.device)
         self.adv_out = torch.empty((nt, n, ny, nx), dtype=torch.float64, device=self.device)
-        self.launches_per_step = FCT_LAUNCHES + remap_launches(nt, n, self.n1, ny * nx)
+        self.launches_per_step = FCT_LAUNCHES + L.pocean_remap_launches(n, self.n1, ny, nx, nt)
 
     def stream(self) -> int:
         return torch.cuda.current_stream(self.device).cuda_stream
