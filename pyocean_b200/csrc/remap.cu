@@ -3,8 +3,8 @@
 // Reference: core/vertical/remap.py — remap_column :306-397, reconstruct :234-294, _average :297-303,
 // _remap_columns :400-415 (one call per field there; here every field of the stack in one launch).
 //
-// Mapping.  Columns of up to SG_LAYERS layers are remapped with their layers side by side (remap_segments_body below).
-// Deeper ones, and large batches of domains: one thread owns one column and NF fields of it; consecutive threads take
+// Mapping.  Columns of up to SG_LAYERS layers are remapped with their layers side by side (remap_segments_body below) where
+// that is faster (remap_form).  Deeper ones, large batches of domains and large planes of few layers: one thread owns one column and NF fields of it; consecutive threads take
 // consecutive i, so each per-layer load or store of a warp is one contiguous 256-byte segment of the (k, j, i) arrays (a warp per column
 // would touch 8 bytes of every 32-byte sector instead).  The column is processed in one pass (remap_core.cuh,
 // remap_column_stream): a 6-cell register window builds each source cell's polynomial from its neighbours and the
@@ -125,9 +125,8 @@ __global__ void __launch_bounds__(128) remap_general_kernel(const double* __rest
 //               behind: integral r belongs to the cell that leaves target r, one thread each, all alike;
 //   residuals   per cell, its integrals summed in the order of the targets;
 //   contents    per target, its pieces summed in the order of the cells.
-// Same arithmetic as the sweep, same results.  Two fields of 360 x 360 x 50 take 0.48 ms against 0.68 by the sweep (0.80
-// before its divisions by 3 were shortened), of 512 x 512 x 50 0.94 against 1.04, one of 150 x 121 x 30 38 us against 100,
-// one of 64 x 64 x 20 13 us against 90; one field of 512 x 512 x 50 0.65 against 0.67, without land 0.74 against 0.68.
+// Same arithmetic as the sweep, same results.  Two fields of 360 x 360 x 50 take 0.53 ms against 0.70 by the sweep, one of
+// 150 x 121 x 30 38 us against 100, one of 64 x 64 x 20 13 us against 90; remap_form says where the sweep is faster.
 constexpr int SG_COLS = 8;
 constexpr int SG_THREADS = 256;                 // most threads of a CTA
 constexpr int SG_LAYERS = 96;
@@ -563,13 +562,6 @@ __global__ void __launch_bounds__(128) reconstruct_kernel(const double* __restri
 
 }  // namespace remap
 
-// Whether a batch of `columns` column-fields of up to nmax layers is remapped with the layers of a column side by side:
-// batches that the one-thread-per-column sweep leaves the chip idle for (it holds 95 000 columns at a time).  Larger ones
-// take the sweep: their domains' depths differ, and the shared memory of the deepest one's columns leaves too few CTAs
-// (24 domains of one tracer: a step's remap 1.98 ms by the sweep, 2.4 ms side by side; 8 domains of 48..160 cells: the
-// two steps 1.71 ms by the sweep, 1.47 ms side by side).
-bool remap_batch_segments(long long columns, int nmax) { return nmax <= remap::SG_LAYERS && columns <= 150000; }
-
 // The most dynamic shared memory a side-by-side launch takes: columns of SG_LAYERS layers of one field; field pairs up to
 // three CTAs an SM.
 constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_LAYERS), SG_SMEM2 = 72 * 1024;
@@ -581,23 +573,67 @@ constexpr size_t SG_SMEM1 = remap::segment_smem(1, remap::SG_LAYERS, remap::SG_L
 // sweep 0.49 and 0.29).
 static bool irregular_launch(long long columns, int n) { return columns * n > 1000000; }
 
-// The launches of a remap: of field pairs and of single fields, side by side or by the sweep, and the irregular columns'.
+// Whether the sweep remaps `columns` columns faster than they are remapped side by side.  It holds a wave of columns at a
+// time; a wave costs it the same whatever is in it but for the last, which costs between half and a whole one, while side by
+// side the time is proportional to the columns, `ratio` times the sweep's for whole waves.
+static bool sweep_pays(long long columns, long long wave, double ratio)
+{
+    const long long full = columns / wave;
+    const double rest = (double)(columns - full * wave) / wave;
+    return ratio * ((double)full + rest) > full + (rest > 0.0 ? 0.5 + 0.5 * rest : 0.0);
+}
+
+// The ratio falls with the layers n, since side by side each column has its barriers whatever its depth.  Side by side / by
+// the sweep, measured for whole waves (1024 x 1024, 724 x 724 and 512 x 512 columns, PPM_H4, us):
+//   field pairs     2 layers 380/136, 4 677/335, 8 880/661, 12 1099/976, 20 1785/1654, 30 685/703, 50 1096/1177;
+//   single fields   2 layers 290/83, 4 419/196, 8 577/390, 12 734/593, 20 1175/1005, 30 480/435, 50 753/734, 96 1562/1422.
+// Pairs above 70 layers, which go side by side as two single fields: 75 layers of 512 x 512 2274/1778, of 300 x 310 822/660,
+// of 240 x 240 517/558, 309 x 309 (just over a wave) 835/974.
+static double side_ratio(int nf, double n)
+{
+    if (nf == 2) return 0.87 + 3.6 / n;
+    return n <= 64 ? 0.95 + 3.0 / n : 1.06;
+}
+constexpr double SIDE_RATIO_DEEP_PAIRS = 1.28;
+constexpr long long SWEEP_WAVE1 = 148 * POCEAN_REMAP1_CTAS * 128, SWEEP_WAVE2 = 148 * POCEAN_REMAP_CTAS * 128;
+
+// Whether a batch of `columns` column-fields of up to nmax layers is remapped with the layers of a column side by side:
+// batches that the one-thread-per-column sweep leaves the chip idle for, unless they are shallow.  Larger ones
+// take the sweep: their domains' depths differ, and the shared memory of the deepest one's columns leaves too few CTAs
+// (24 domains of one tracer: a step's remap 1.98 ms by the sweep, 2.4 ms side by side; 8 domains of 48..160 cells: the
+// two steps 1.71 ms by the sweep, 1.47 ms side by side).
+bool remap_batch_segments(long long columns, int nmax)
+{
+    return nmax <= remap::SG_LAYERS && columns <= 150000 &&
+           !(nmax <= 16 && sweep_pays(columns, SWEEP_WAVE1, side_ratio(1, nmax)));
+}
+
+// The launches of a remap: of field pairs and of single fields, each side by side or by the sweep, and the irregular
+// columns'.  Side by side, two fields of a column share the work on its thicknesses while three CTAs fit an SM.
 struct RemapForm {
     int pairs, singles;
-    bool side, general;
+    bool side_pairs, side_singles, general;
     int launches() const { return (pairs > 0) + (singles > 0) + general; }
 };
 
-// Side by side, two fields of a column share the work on its thicknesses while three CTAs fit an SM.  Where they do not
-// (above 70 layers) and the columns fill the chip, the sweep's field pairs are faster: two fields of 512 x 512 x 75
-// take 0.79 ms as two single fields side by side, 0.62 by the sweep; 60 x 60 x 75 with four 24 us against 176.
 static RemapForm remap_form(int n0, int n1, i64 plane, int nfields)
 {
     const int mx = n0 > n1 ? n0 : n1;
+    const double n = 0.5 * (n0 + n1);
+    RemapForm f{nfields / 2, nfields % 2, false, false, true};
+    if (mx > remap::SG_LAYERS) return f;
     const bool fit2 = remap::segment_smem(2, n0, n1) <= SG_SMEM2;
-    if (mx > remap::SG_LAYERS || !(fit2 || nfields == 1 || plane < 150000)) return {nfields / 2, nfields % 2, false, true};
-    const int pairs = fit2 ? nfields / 2 : 0;
-    return {pairs, nfields - 2 * pairs, true, irregular_launch((long long)plane * nfields, mx)};
+    f.side_pairs = f.pairs && !sweep_pays(plane * f.pairs, SWEEP_WAVE2, fit2 ? side_ratio(2, n) : SIDE_RATIO_DEEP_PAIRS);
+    if (f.side_pairs && !fit2) {
+        f.pairs = 0;
+        f.singles = nfields;
+        f.side_singles = true;
+    } else {
+        f.side_singles = f.singles && !sweep_pays(plane, SWEEP_WAVE1, side_ratio(1, n));
+    }
+    f.general = (f.pairs && !f.side_pairs) || (f.singles && !f.side_singles) ||
+                irregular_launch((long long)plane * nfields, mx);
+    return f;
 }
 
 // Columns of a batched remap CTA.
@@ -694,47 +730,35 @@ extern "C" int pocean_remap_columns_f64(const double* h_src, const double* f_src
     cudaStream_t st = (cudaStream_t)stream;
     const i64 plane = (i64)ny * nx;
     const RemapForm form = remap_form(n0, n1, plane, nfields);
-    if (form.side) {
-        const int nf2 = form.pairs, rest = form.singles;
-        const int threads = remap::segment_threads(n0, n1);
-        const dim3 g((unsigned)((plane + remap::SG_COLS - 1) / remap::SG_COLS), (unsigned)nf2);
-        const size_t s1 = remap::segment_smem(1, n0, n1), s2 = remap::segment_smem(2, n0, n1);
-        const bool mark = form.general, five = s1 <= remap::SG_FIVE;
-        const auto one = mark ? (five ? remap::remap_segments_kernel<1, 5, true> : remap::remap_segments_kernel<1, 4, true>)
-                              : (five ? remap::remap_segments_kernel<1, 5, false>
-                                      : remap::remap_segments_kernel<1, 4, false>);
-        const auto two = mark ? remap::remap_segments_kernel<2, 4, true> : remap::remap_segments_kernel<2, 4, false>;
-        cudaError_t e = rest ? allow_smem((const void*)one, SG_SMEM1) : cudaSuccess;
-        if (e == cudaSuccess && nf2) e = allow_smem((const void*)two, SG_SMEM2);
-        if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
-        if (nf2) two<<<g, threads, s2, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 0, scheme, out);
-        if (rest)
-            one<<<dim3(g.x, (unsigned)rest), threads, s1, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 2 * nf2, scheme,
-                                                                out);
-        if (mark) remap_general_launch(h_src, f_src, h_tgt, n0, n1, plane, nfields, scheme, out, st);
-        return pocean_check_launch(fn);
-    }
-    const unsigned gx = (unsigned)((plane + 127) / 128);
-    const int pairs = form.pairs;
+    const int pairs = form.pairs, singles = form.singles, threads = remap::segment_threads(n0, n1);
+    const unsigned side = (unsigned)((plane + remap::SG_COLS - 1) / remap::SG_COLS), gx = (unsigned)((plane + 127) / 128);
     // 32-bit offsets within a field when every field (n0 or n1 layers of the plane) holds fewer than 2^31 entries
     const bool small = (i64)(n0 > n1 ? n0 : n1) * plane < (1ll << 31);
-    if (pairs > 0) {
-        if (small)
-            remap::remap_stream_kernel<2, int><<<dim3(gx, pairs), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1,
-                                                                                plane, 0, scheme, out);
-        else
-            remap::remap_stream_kernel<2, i64><<<dim3(gx, pairs), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1,
-                                                                                plane, 0, scheme, out);
+    if (pairs > 0 && form.side_pairs) {
+        const auto kernel = form.general ? remap::remap_segments_kernel<2, 4, true> : remap::remap_segments_kernel<2, 4, false>;
+        const cudaError_t e = allow_smem((const void*)kernel, SG_SMEM2);
+        if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
+        kernel<<<dim3(side, (unsigned)pairs), threads, remap::segment_smem(2, n0, n1), st>>>(
+            h_src, f_src, h_tgt, wet, n0, n1, plane, 0, scheme, out);
+    } else if (pairs > 0) {
+        const auto kernel = small ? remap::remap_stream_kernel<2, int> : remap::remap_stream_kernel<2, i64>;
+        kernel<<<dim3(gx, (unsigned)pairs), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 0, scheme, out);
     }
-    if (form.singles) {
-        if (small)
-            remap::remap_stream_kernel<1, int><<<dim3(gx, 1), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane,
-                                                                            nfields - 1, scheme, out);
-        else
-            remap::remap_stream_kernel<1, i64><<<dim3(gx, 1), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane,
-                                                                            nfields - 1, scheme, out);
+    if (singles > 0 && form.side_singles) {
+        const size_t s1 = remap::segment_smem(1, n0, n1);
+        const bool five = s1 <= remap::SG_FIVE;
+        const auto kernel = form.general
+                                ? (five ? remap::remap_segments_kernel<1, 5, true> : remap::remap_segments_kernel<1, 4, true>)
+                                : (five ? remap::remap_segments_kernel<1, 5, false> : remap::remap_segments_kernel<1, 4, false>);
+        const cudaError_t e = allow_smem((const void*)kernel, SG_SMEM1);
+        if (e != cudaSuccess) return pocean_fail(POCEAN_ECUDA, "%s: %s", fn, cudaGetErrorString(e));
+        kernel<<<dim3(side, (unsigned)singles), threads, s1, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 2 * pairs, scheme,
+                                                                   out);
+    } else if (singles > 0) {
+        const auto kernel = small ? remap::remap_stream_kernel<1, int> : remap::remap_stream_kernel<1, i64>;
+        kernel<<<dim3(gx, (unsigned)singles), 128, 0, st>>>(h_src, f_src, h_tgt, wet, n0, n1, plane, 2 * pairs, scheme, out);
     }
-    remap_general_launch(h_src, f_src, h_tgt, n0, n1, plane, nfields, scheme, out, st);
+    if (form.general) remap_general_launch(h_src, f_src, h_tgt, n0, n1, plane, nfields, scheme, out, st);
     return pocean_check_launch(fn);
 }
 

@@ -84,3 +84,14 @@ def test_batched_irregular_columns(side):
         with np.errstate(all="ignore"):
             for m in range(c.shape[0]):
                 np.testing.assert_array_equal(got[m], O.remap_columns(w.h_src, c[m], w.h_tgt, w.remap_scheme, w.wet))
+
+
+# planes that go by the sweep, side by side, or the pairs one way and the odd field the other
+@pytest.mark.parametrize("n,ny,nx,nf", [(1, 150, 140, 1), (2, 150, 150, 3), (3, 200, 200, 3), (10, 300, 310, 3), (30, 300, 310, 3),
+                                        (12, 362, 363, 3), (75, 262, 262, 3), (75, 240, 240, 3)])
+def test_around_the_sweep(n, ny, nx, nf):
+    hs, f, ht, wet = _columns(n, n, n, ny, nx, nf)
+    with np.errstate(all="ignore"):
+        got = P.remap_columns(hs, f, ht, P.PPM_H4, wet)
+        for m in range(nf):
+            np.testing.assert_array_equal(got[m], O.remap_columns(hs, f[m], ht, P.PPM_H4, wet))
