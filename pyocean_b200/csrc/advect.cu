@@ -715,7 +715,7 @@ __device__ __forceinline__ double zface_lin(const StepArgs& a, const Shape& s, c
 // cells), took 6.68 ms at 512 x 512 x 50 with a vertical transport; these passes take 3.86 ms, bit-identical.
 // Stages 1-3: SSP-RK3 (input C, c1, c2); 4: the 'pc' predictor (input C, centred faces, half step to c1); 5: the
 // 'pc' corrector (input c1, the scheme's faces, full step from C); 0: one evaluation of C's faces.  The WENO5 faces of
-// the steps read their stencils' classes from `cls` (rk3_class_kernel); the single evaluation works its own out.
+// the steps read their stencils' classes from `cls` (rk3_class_kernel); the single evaluation works out those it takes.
 template <int STAGE>
 __device__ __forceinline__ const double* rk3_stage_field(const StepArgs& a)
 {
@@ -747,6 +747,27 @@ __device__ __forceinline__ void rk3_lin_faces(const StepArgs& a, int t, int k, i
     if (j == s.ny - 1) sy[fyo + s.nx] = y_face_lin<FS>(P, s, fl, s.ny, i);
 }
 
+// The class of a face's upwind stencil alone (face_class's bits of its direction), for a single evaluation.
+__device__ __forceinline__ unsigned upwind_class(const uint8_t* __restrict__ ok, int st, int n, bool per, int f, double q)
+{
+    const bool pos = q >= 0.0;
+    const int g0 = pos ? f - 3 : f + 2, dg = pos ? 1 : -1;
+    bool v[5];
+    if (f >= 3 && f + 2 < n) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) v[m] = __ldg(ok + (g0 + m * dg) * st) != 0;
+    } else {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+            int g = g0 + m * dg;
+            bool in = true;
+            if (per) g = wrap(g, n); else in = g >= 0 && g < n;
+            v[m] = in && __ldg(ok + (in ? g : 0) * st) != 0;
+        }
+    }
+    return stencil_class(v[0], v[1], v[2], v[3], v[4]) << (pos ? 0 : 2);
+}
+
 // The WENO5 faces of cell (k, j, i) for tracers t0 .. t1-1; INNER: at least three cells from every horizontal edge (see
 // faces_cell).
 template <int STAGE, bool ZV, bool INNER>
@@ -757,13 +778,19 @@ __device__ __forceinline__ void rk3_weno_faces(const StepArgs& a, const uint16_t
     const Flags fl(a.flags);
     const int pl = s.ny * s.nx, xpl = s.ny * (s.nx + 1), ypl = (s.ny + 1) * s.nx;
     const int o = j * s.nx + i, ox = o + j;
-    const unsigned cls = STAGE == 0 ? rk3_classes(a, s, fl, k, j, i) : __ldg(classes + plane_at(k, pl) + o);
+    unsigned cls = STAGE == 0 ? 0u : __ldg(classes + plane_at(k, pl) + o);
     const double* __restrict__ qx = a.Qx + plane_at(k, xpl);
     const double* __restrict__ qy = a.Qy + plane_at(k, ypl);
     const double qw = __ldg(qx + ox), qs = __ldg(qy + o);
     // bottom interface: between layers k - 1 and k of the column, 0 on the bed (sigma_baroclinic.py:335-353)
     const double qb = a.Fz != nullptr && k >= 1 ? __ldg(a.Fz + plane_at(k, pl) + o) : 0.0;
     const bool per_x = !INNER && fl.per_x, per_y = !INNER && fl.per_y;
+    if (STAGE == 0) {
+        const uint8_t* ok = a.ok + plane_at(k, pl);
+        if (qw != 0.0) cls = upwind_class(ok + j * s.nx, 1, s.nx, per_x, i, qw);
+        if (qs != 0.0) cls |= upwind_class(ok + i, s.nx, s.ny, per_y, j, qs) << 4;
+        if (qb != 0.0) cls |= upwind_class(a.ok + o, pl, s.n, false, k, qb) << 8;
+    }
 #pragma unroll 1
     for (int t = t0; t < t1; ++t) {
         const int p = t * s.n + k;

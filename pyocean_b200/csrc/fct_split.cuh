@@ -45,6 +45,11 @@ __device__ __forceinline__ unsigned face_class(const bool* v)
 __device__ __forceinline__ unsigned line_class(const uint8_t* __restrict__ ok, int st, int n, bool per, int f)
 {
     bool v[6];
+    if (f >= 3 && f + 2 < n) {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) v[m] = __ldg(ok + (f - 3 + m) * st) != 0;
+        return face_class(v);
+    }
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
         int g = f - 3 + m;
