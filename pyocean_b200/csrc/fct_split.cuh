@@ -101,7 +101,7 @@ __device__ __forceinline__ unsigned class4(const unsigned* v)
 // depend on ok alone), one byte per cell; the face passes used to load and test five ok bytes per stencil.  A thread
 // takes four neighbouring cells, their validity in the bytes of a word; where nx is a multiple of four and ok starts
 // on a word, rows are read and written by words.
-// Bounded by instruction issue (72 %): 31 us at 512 x 512 x 50, where the face passes it serves went from 2.11 to 1.47 ms
+// Bounded by instruction issue (71 %): 39 us at 512 x 512 x 50, where the face passes it serves went from 2.11 to 1.47 ms
 // (with their shorter divisions and tracer loop).  64 uneven boxes: 1.06 ms with rows that start off a word read by bytes,
 // 0.84 so; two or four rows a thread were within the noise of one.
 __device__ __forceinline__ void class_body(const StepArgs& a, int k, int i, int j)
